@@ -240,7 +240,7 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
         extern __shared__ __align__(16) unsigned char s_heaps[];
         const int wbase = gtid & ~31;
         CoopLane W(C, wbase);
-        W.sheap = reinterpret_cast<WinEntry*>(s_heaps);
+        W.sheap = reinterpret_cast<HeapEntry*>(s_heaps);
         for (;;) {
             int rc = 0;
             if ((threadIdx.x & 31) == 0) rc = atomicAdd(O.coop_work, 1);
@@ -262,7 +262,7 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
     int waited = 0;
     int adopt = -1;
     for (;;) {
-        const int act = v >= 0 ? L.template peek<SVG_ICH_INLINE_STALE>() : -1;
+        const int act = v >= 0 ? L.template take<SVG_ICH_INLINE_STALE>() : -1;
         const unsigned m0 = __ballot_sync(kFull, act == Lane::kActWindow);
         const unsigned m1 = __ballot_sync(kFull, act == Lane::kActPseudo);
         const unsigned m2 = __ballot_sync(kFull, act == Lane::kActDone);
@@ -285,10 +285,8 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
         if (chosen == Lane::kActDone) finish_warp(L, O, v, amask);  // the whole warp exports
         if (act == chosen) {
             waited = 0;
-            if (chosen == Lane::kActWindow) {
-                L.act_window(amask);
-            } else if (chosen == Lane::kActPseudo) {
-                L.act_pseudo(amask);
+            if (chosen != Lane::kActDone) {
+                L.act(chosen, amask);
             } else {
                 r = O.coop_n + atomicAdd(O.work, 1);
                 v = r < O.nsrc ? O.order[r] : -1;
@@ -607,10 +605,10 @@ int trace_blocks(int64_t nnz) { return (int)std::max<int64_t>(1, std::min<int64_
 
 size_t lane_bytes(const Layout& l) {
     size_t b = 0;
-    b += (size_t)heap_stride(l.wphys) * sizeof(WinEntry);
+    b += (size_t)heap_stride(l.wphys) * sizeof(HeapEntry);
     b += (size_t)l.wphys * sizeof(WinPay);
     b += (size_t)l.wphys * sizeof(uint16_t);
-    b += (size_t)heap_stride(l.pphys) * sizeof(PsEntry);
+    b += (size_t)heap_stride(l.pphys) * sizeof(HeapEntry);
     b += ((size_t)1 << l.vcap_log2) * sizeof(VSlot);
     b += (size_t)l.vlimit * sizeof(int32_t);
     b += ((size_t)1 << l.scap_log2) * sizeof(SSlot);
@@ -629,10 +627,10 @@ Arena g_arena[2];  // [0] main pass, [1] retry pass with larger tables
 void carve(Arena& A, const Layout& l, LaneConfig& C, cudaStream_t st) {
     size_t lanes = (size_t)l.lanes;
     size_t sz[7] = {
-        align_up(lanes * heap_stride(l.wphys) * sizeof(WinEntry)),
+        align_up(lanes * heap_stride(l.wphys) * sizeof(HeapEntry)),
         align_up(lanes * l.wphys * sizeof(WinPay)),
         align_up(lanes * l.wphys * sizeof(uint16_t)),
-        align_up(lanes * heap_stride(l.pphys) * sizeof(PsEntry)),
+        align_up(lanes * heap_stride(l.pphys) * sizeof(HeapEntry)),
         align_up(lanes * ((size_t)1 << l.vcap_log2) * sizeof(VSlot)),
         align_up(lanes * l.vlimit * sizeof(int32_t)),
         align_up(lanes * ((size_t)1 << l.scap_log2) * sizeof(SSlot)),
@@ -643,10 +641,10 @@ void carve(Arena& A, const Layout& l, LaneConfig& C, cudaStream_t st) {
     bool fresh = !(A.layout == l) || A.buf.bytes < total;
     if (A.buf.bytes < total) A.buf.reserve(total);
     char* p = A.buf.as<char>();
-    C.wheap = reinterpret_cast<WinEntry*>(p); p += sz[0];
+    C.wheap = reinterpret_cast<HeapEntry*>(p); p += sz[0];
     C.wpool = reinterpret_cast<WinPay*>(p); p += sz[1];
     C.wfree = reinterpret_cast<uint16_t*>(p); p += sz[2];
-    C.pheap = reinterpret_cast<PsEntry*>(p); p += sz[3];
+    C.pheap = reinterpret_cast<HeapEntry*>(p); p += sz[3];
     C.vtab = reinterpret_cast<VSlot*>(p); p += sz[4];
     C.vlist = reinterpret_cast<int32_t*>(p); p += sz[5];
     C.stab = reinterpret_cast<SSlot*>(p); p += sz[6];
@@ -1090,6 +1088,13 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     } else if (blocks <= 0) {
         int per_sm = 0;
         SVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ich_batched, tpb, 0));
+        // A third block per SM raises the throughput but also the time of each
+        // lane's step, and with few sources per lane the heaviest sources' steps
+        // are the build's length.  Measured, two blocks against three: 73K
+        // sources (1.3 per lane of three blocks) 31.0 / 32.2 ms at K = 100 and
+        // 455 / 530 ms at K = 500; 120K sources (2.1) 51.1 / 42.0 ms at K = 100
+        // and 162 / 140 ms at K = 200; 750K sources 277 / 240 ms at K = 100.
+        if (per_sm > 2 && 4 * (int64_t)nsrc < (int64_t)7 * per_sm * prop.multiProcessorCount * tpb) per_sm = 2;
         blocks = std::max(1, per_sm) * prop.multiProcessorCount;
     }
     int64_t want_blocks = (nsrc + tpb - 1) / tpb;
@@ -1249,7 +1254,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
             O.cand_start = b_candstart.as<int64_t>();
             // the cooperative warps' heaps: window then pseudo-source entries
             const size_t coop_smem =
-                coop_warps > 0 ? ((size_t)C.wstride * sizeof(WinEntry) + (size_t)C.pstride * sizeof(PsEntry)) : 0;
+                coop_warps > 0 ? ((size_t)C.wstride * sizeof(HeapEntry) + (size_t)C.pstride * sizeof(HeapEntry)) : 0;
             if (coop_smem > 48 * 1024)
                 SVG_CUDA(cudaFuncSetAttribute(k_ich_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)coop_smem));
@@ -1644,10 +1649,10 @@ constexpr int kStaticSlimit = (3 << kStaticScapLog2) / 4;
 
 constexpr size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 constexpr int kStaticStride = (kStaticWcap + 16 + 3) / 4 * 4;  // heap entries per lane
-constexpr size_t kSzWheap = al256((size_t)kStaticLanes * kStaticStride * sizeof(WinEntry));
+constexpr size_t kSzWheap = al256((size_t)kStaticLanes * kStaticStride * sizeof(HeapEntry));
 constexpr size_t kSzWpool = al256((size_t)kStaticLanes * kStaticWcap * sizeof(WinPay));
 constexpr size_t kSzWfree = al256((size_t)kStaticLanes * kStaticWcap * sizeof(uint16_t));
-constexpr size_t kSzPheap = al256((size_t)kStaticLanes * kStaticStride * sizeof(PsEntry));
+constexpr size_t kSzPheap = al256((size_t)kStaticLanes * kStaticStride * sizeof(HeapEntry));
 constexpr size_t kSzVtab = al256((size_t)kStaticLanes * ((size_t)1 << kStaticVcapLog2) * sizeof(VSlot));
 constexpr size_t kSzVlist = al256((size_t)kStaticLanes * kStaticVlimit * sizeof(int32_t));
 constexpr size_t kSzStab = al256((size_t)kStaticLanes * ((size_t)1 << kStaticScapLog2) * sizeof(SSlot));
@@ -1757,10 +1762,10 @@ extern "C" svg_status svg_build_rows_static(svg_mesh* m, int32_t K, int32_t sour
         C.slimit = kStaticSlimit;
         C.watchdog = (int64_t)1 << 26;
         char* p = base;
-        C.wheap = reinterpret_cast<WinEntry*>(p); p += kSzWheap;
+        C.wheap = reinterpret_cast<HeapEntry*>(p); p += kSzWheap;
         C.wpool = reinterpret_cast<WinPay*>(p); p += kSzWpool;
         C.wfree = reinterpret_cast<uint16_t*>(p); p += kSzWfree;
-        C.pheap = reinterpret_cast<PsEntry*>(p); p += kSzPheap;
+        C.pheap = reinterpret_cast<HeapEntry*>(p); p += kSzPheap;
         C.vtab = reinterpret_cast<VSlot*>(p); p += kSzVtab;
         C.vlist = reinterpret_cast<int32_t*>(p); p += kSzVlist;
         C.stab = reinterpret_cast<SSlot*>(p); p += kSzStab;

@@ -39,56 +39,10 @@
 
 #include "svg_internal.h"
 
+// Outdated heap tops a lane of the batched kernel drops inside one take()
+// (16 measured 0.1-0.4 % slower)
 #ifndef SVG_ICH_INLINE_STALE
 #define SVG_ICH_INLINE_STALE 8
-#endif
-// 1: the one-thread sifts prefetch keys only and re-read the moved entries;
-// 0: they prefetch whole entries (one L1 round trip fewer per move).  With the
-// three-level sift-down below, keys only measured 1.3 % faster (the sift-up
-// holds fewer registers)
-#ifndef SVG_KEYS_ONLY_SIFT
-#define SVG_KEYS_ONLY_SIFT 1
-#endif
-// keys-only sift-up: ancestors whose keys are read in one round trip
-#ifndef SVG_UP_LEVELS
-#define SVG_UP_LEVELS 4
-#endif
-// 1: the keys-only sift-up reads a further batch of ancestors' keys per round
-// trip while the climb goes on (0: one level per round trip past the first batch)
-#ifndef SVG_UP_BATCHES
-#define SVG_UP_BATCHES 1
-#endif
-// keys-only sift-up: up to this many ancestors, the moved entries are read
-// into registers together and then written; beyond it, one at a time
-#ifndef SVG_UP_ARRAY
-#define SVG_UP_ARRAY 4
-#endif
-// 1: the one-thread sift-down reads the keys of three levels per round trip
-// (measured 2.6 % faster on the 72.9K height field at K = 500, 4 % on the
-// 750K torus)
-#ifndef SVG_SIFT3
-#define SVG_SIFT3 1
-#endif
-// 1: the free pool slot on top of the lane's free list is kept in a register,
-// so a push does not wait for the list read (measured 1-1.5 % faster)
-#ifndef SVG_FREE_CACHE
-#define SVG_FREE_CACHE 1
-#endif
-// 1: a lane's counters and its cached look at the heap tops live in shared
-// memory (one slot per thread, structure of arrays) instead of registers
-// (measured 3-4 % faster)
-#ifndef SVG_SMEM_STATE
-#define SVG_SMEM_STATE 1
-#endif
-// 1: propagate() inserts a missing vertex or split entry at the empty slot its
-// lookup ended on (no second probe walk; measured 2-4.5 % faster)
-#ifndef SVG_INSERT_AT
-#define SVG_INSERT_AT 1
-#endif
-// 1: propagate() builds, tests and pushes one child window at a time through
-// one copy of the code (fewer live registers; measured 10 % faster)
-#ifndef SVG_SEQ_CHILD
-#define SVG_SEQ_CHILD 1
 #endif
 
 namespace svgb {
@@ -105,10 +59,14 @@ enum : int32_t {
     kFlagCapacity = 16,     // this lane's tables filled: the source is re-run with bigger ones
 };
 
-struct alignas(16) WinEntry {
-    double key;     // window minDist
-    int32_t psrc;   // pseudo-source vertex
-    uint32_t sb;    // pool slot (low 16 bits) | birth (bits 16..23)
+// Entry of a lane's two heaps.
+//   window heap:        key = window minDist, id = pseudo-source vertex,
+//                       bits = pool slot (low 16 bits) | birth (bits 16..23)
+//   pseudo-source heap: key = its distance, id = vertex, bits = level << 8 | birth
+struct alignas(16) HeapEntry {
+    double key;
+    int32_t id;
+    uint32_t bits;
 };
 struct alignas(16) WinPay {
     double b0, b1;  // interval on the half-edge
@@ -116,11 +74,6 @@ struct alignas(16) WinPay {
     double psd;     // pseudoSrcDist
     int32_t cross;  // twin of the window's half-edge: where it propagates (-1: boundary)
     int32_t level;
-};
-struct alignas(16) PsEntry {
-    double key;     // pseudo-source distance
-    int32_t vert;
-    uint32_t lb;    // level << 8 | birth
 };
 struct alignas(32) VSlot {
     uint32_t key;
@@ -166,10 +119,10 @@ struct LaneConfig {
     int32_t vlimit, slimit;  // max keys this lane's tables take before kFlagCapacity
     int64_t watchdog;        // max steps per source
     int32_t max_wait;        // batched kernel: most iterations a lane waits for the vote to pick its step
-    WinEntry* wheap;
+    HeapEntry* wheap;
     WinPay* wpool;
     uint16_t* wfree;
-    PsEntry* pheap;
+    HeapEntry* pheap;
     VSlot* vtab;
     int32_t* vlist;
     SSlot* stab;
@@ -184,7 +137,7 @@ __device__ __forceinline__ HeRec ld_he(const HeRec* p, int e) {
     int4 a = __ldg(q);
     int4 b = __ldg(q + 1);
     HeRec h;
-    h.v0 = a.x; h.v1 = a.y; h.twin = a.z; h.pad = a.w;
+    h.v0 = a.x; h.v1 = a.y; h.twin = a.z; h.vflags = a.w;
     h.len = __hiloint2double(b.y, b.x);
     h.corner = __hiloint2double(b.w, b.z);
     return h;
@@ -330,21 +283,42 @@ __device__ __forceinline__ ProbeQ probe_off() {
     return q;
 }
 
-#if SVG_SMEM_STATE
 // Per-thread slots (blocks of up to 128 threads) of the lane state that a
-// step touches once or twice: counters and the cached heap tops.
+// step touches once or twice: counters, the popped heap entry waiting for its
+// action, and that entry's window payload, fetched by an asynchronous copy
+// that overlaps the pop's sift-down (no register holds it meanwhile).
 struct LaneSmem {
-    double wkey[128];
-    int32_t wpsrc[128];
-    uint32_t wsb[128];
+    int4 pay[3][128];
     double pkey[128];
-    int32_t pvert[128];
-    uint32_t plb[128];
+    int32_t pid[128];
+    uint32_t pbits[128];
     int32_t windows[128], pseudos[128], generated[128], maxw[128], maxp[128];
     long long steps[128];
 };
 __shared__ LaneSmem g_lane_smem;
-#endif
+
+// 16 bytes from global to shared memory without a register in between.
+__device__ __forceinline__ void copy_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)),
+                 "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// a / b - 1 > kRelErr as the reference computes it (ICHDevice.cu:952, 668),
+// for a > b: outside a band around b (1 + kRelErr) far wider than the three
+// roundings involved the comparison decides, and only inside it is the
+// division done.  A warp would otherwise wait for it at nearly every window.
+__device__ __forceinline__ bool exceeds_rel(double a, double b) {
+    if (a >= b * (1.0 + 1.01 * kRelErr)) return b >= 0.0;  // a negative b gives a ratio below 1
+    if (a <= b * (1.0 + 0.99 * kRelErr)) return false;
+    return a / b - 1.0 > kRelErr;
+}
+// a > b and a / b - 1 > 0 (ICHDevice.cu:927-933).  For b > 0 the next double
+// after b = m 2^e (1 <= m < 2) is b (1 + 2^-52 / m), and 2^-52 / m > 2^-53, so
+// the quotient of any a > b rounds above 1 and the comparison is the whole
+// test (a / 0 is infinite); a negative b gives a quotient below 1.
+__device__ __forceinline__ bool exceeds(double a, double b) { return a > b && b >= 0.0; }
 
 template <bool kCoop>
 struct LaneT {
@@ -355,15 +329,15 @@ struct LaneT {
     // The cooperative form keeps its source's two heaps in shared memory
     // (sheap: wstride window entries, then pstride pseudo-source entries), or,
     // for a source it adopted from a lane (sheap null), in that lane's scratch.
-    WinEntry* sheap = nullptr;
-    __device__ __forceinline__ WinEntry* WH() const {
+    HeapEntry* sheap = nullptr;
+    __device__ __forceinline__ HeapEntry* WH() const {
         if constexpr (kCoop)
             if (sheap) return sheap;
         return C.wheap + (size_t)lid * C.wstride;
     }
-    __device__ __forceinline__ PsEntry* PH() const {
+    __device__ __forceinline__ HeapEntry* PH() const {
         if constexpr (kCoop)
-            if (sheap) return reinterpret_cast<PsEntry*>(sheap + C.wstride);
+            if (sheap) return sheap + C.wstride;
         return C.pheap + (size_t)lid * C.pstride;
     }
     __device__ __forceinline__ WinPay* WP() const { return C.wpool + (size_t)lid * C.wphys; }
@@ -372,36 +346,31 @@ struct LaneT {
     __device__ __forceinline__ int32_t* VL() const { return C.vlist + (size_t)lid * C.vlimit; }
     __device__ __forceinline__ SSlot* ST() const { return C.stab + ((size_t)lid << C.scap_log2); }
     int wsize, psize, nfree, nfresh;
-    int ftop;       // WF()[nfree - 1] when nfree > 0 (free-slot cache)
+    int ftop;       // WF()[nfree - 1] when nfree > 0: a push does not wait for the list read
     int vcount, scount;
     uint32_t epoch;
     int source;
     int src_birth;
     int total;      // totalCalcVertNum
     int flags;
-#if SVG_SMEM_STATE
+    // The next action, decided and popped by take(), until act() runs it.
+    bool pk_valid;
+    bool pk_proc;   // process (true) or an outdated entry already dropped (false)
+    bool pk_init;   // the source's own first fan (Initialize)
+    int pk_act;
+    bool done;
     __device__ __forceinline__ int& st_windows() const { return g_lane_smem.windows[threadIdx.x]; }
     __device__ __forceinline__ int& st_pseudos() const { return g_lane_smem.pseudos[threadIdx.x]; }
     __device__ __forceinline__ int& st_generated() const { return g_lane_smem.generated[threadIdx.x]; }
     __device__ __forceinline__ int& st_maxw() const { return g_lane_smem.maxw[threadIdx.x]; }
     __device__ __forceinline__ int& st_maxp() const { return g_lane_smem.maxp[threadIdx.x]; }
     __device__ __forceinline__ long long& st_steps() const { return g_lane_smem.steps[threadIdx.x]; }
-#else
-    int windows_, pseudos_, generated_, maxw_, maxp_;
-    long long steps_;
-    __device__ __forceinline__ int& st_windows() { return windows_; }
-    __device__ __forceinline__ int& st_pseudos() { return pseudos_; }
-    __device__ __forceinline__ int& st_generated() { return generated_; }
-    __device__ __forceinline__ int& st_maxw() { return maxw_; }
-    __device__ __forceinline__ int& st_maxp() { return maxp_; }
-    __device__ __forceinline__ long long& st_steps() { return steps_; }
-    __device__ __forceinline__ int st_windows() const { return windows_; }
-    __device__ __forceinline__ int st_pseudos() const { return pseudos_; }
-    __device__ __forceinline__ int st_generated() const { return generated_; }
-    __device__ __forceinline__ int st_maxw() const { return maxw_; }
-    __device__ __forceinline__ int st_maxp() const { return maxp_; }
-    __device__ __forceinline__ long long st_steps() const { return steps_; }
-#endif
+    __device__ __forceinline__ void set_pending(double key, int32_t id, uint32_t bits) const {
+        const int t = threadIdx.x;
+        g_lane_smem.pkey[t] = key;
+        g_lane_smem.pid[t] = id;
+        g_lane_smem.pbits[t] = bits;
+    }
 
     // gtid: the thread's global index (one-thread form) or the warp's first
     // thread's (cooperative form: the warp uses that thread's scratch).
@@ -412,9 +381,8 @@ struct LaneT {
 
     // Cooperative form: take over the source lane o of this warp is running
     // in the one-thread form (every thread calls it; the state comes from
-    // lane o by shuffles, the scratch and heaps stay lane o's).  The adopted
-    // source continues exactly where the lane stood: the next step re-reads
-    // the heap tops the lane's cached look was taken from.
+    // lane o by shuffles, the scratch and heaps stay lane o's, and the action
+    // lane o has pending becomes the warp's).
     template <class Other>
     __device__ void adopt(const Other& L, int o) {
         constexpr unsigned kFull = 0xFFFFFFFFu;
@@ -432,26 +400,34 @@ struct LaneT {
         src_birth = __shfl_sync(kFull, L.src_birth, o);
         total = __shfl_sync(kFull, L.total, o);
         flags = __shfl_sync(kFull, L.flags, o);
-        // (with SVG_SMEM_STATE both lanes' counters are this thread's slot:
-        // each thread reads its slot, the shuffle syncs, each writes its slot)
-        const int sw = __shfl_sync(kFull, L.st_windows(), o);
-        const int sp = __shfl_sync(kFull, L.st_pseudos(), o);
-        const int sg = __shfl_sync(kFull, L.st_generated(), o);
-        const int smw = __shfl_sync(kFull, L.st_maxw(), o);
-        const int smp = __shfl_sync(kFull, L.st_maxp(), o);
-        const long long sst = __shfl_sync(kFull, L.st_steps(), o);
+        done = __shfl_sync(kFull, (int)L.done, o) != 0;
+        pk_valid = __shfl_sync(kFull, (int)L.pk_valid, o) != 0;
+        pk_proc = __shfl_sync(kFull, (int)L.pk_proc, o) != 0;
+        pk_init = __shfl_sync(kFull, (int)L.pk_init, o) != 0;
+        pk_act = __shfl_sync(kFull, L.pk_act, o);
+        // the slots of lane o, read by every thread before any writes its own
+        copy_async_wait();
+        __syncwarp();
+        const int t = (threadIdx.x & ~31) + o;
+        const LaneSmem& G = g_lane_smem;
+        const int sw = G.windows[t], sp = G.pseudos[t], sg = G.generated[t], smw = G.maxw[t], smp = G.maxp[t];
+        const long long sst = G.steps[t];
+        const double k = G.pkey[t];
+        const int32_t id = G.pid[t];
+        const uint32_t bits = G.pbits[t];
+        const int4 p0 = G.pay[0][t], p1 = G.pay[1][t], p2 = G.pay[2][t];
+        __syncwarp();
         st_windows() = sw;
         st_pseudos() = sp;
         st_generated() = sg;
         st_maxw() = smw;
         st_maxp() = smp;
         st_steps() = sst;
-        done = __shfl_sync(kFull, (int)L.done, o) != 0;
-        pk_valid = false;
+        set_pending(k, id, bits);
+        g_lane_smem.pay[0][threadIdx.x] = p0;
+        g_lane_smem.pay[1][threadIdx.x] = p1;
+        g_lane_smem.pay[2][threadIdx.x] = p2;
     }
-
-    __device__ __forceinline__ WinEntry& wh(int i) { return WH()[i]; }
-    __device__ __forceinline__ PsEntry& ph(int i) { return PH()[i]; }
 
     // ---------------------------------------------------------- tables
     __device__ __forceinline__ uint32_t vhash(uint32_t k) const { return (k * 0x9E3779B1u) >> (32 - C.vcap_log2); }
@@ -464,17 +440,6 @@ struct LaneT {
         return r0;
     }
 
-    // slot index of vertex v, or -1 if absent
-    __device__ __forceinline__ int vfind(int v) {
-        if constexpr (kCoop) return probe1(VT(), C.vcap_log2, (uint32_t)v).slot;
-        uint32_t mask = (1u << C.vcap_log2) - 1, h = vhash((uint32_t)v);
-        for (;;) {
-            uint2 ke = *reinterpret_cast<const uint2*>(&VT()[h]);
-            if (ke.y != epoch) return -1;
-            if (ke.x == (uint32_t)v) return (int)h;
-            h = (h + 1) & mask;
-        }
-    }
     // First probe of a lookup, issued without waiting: slot key/epoch/enter/birth
     // and the distance (one 32-byte sector).  vfinish completes the probe chain.
     __device__ __forceinline__ void vfirst(int v, uint32_t& h, int4& k, double& d) const {
@@ -493,6 +458,33 @@ struct LaneT {
             d = VT()[h].dist;
         }
     }
+    // Slot of vertex v or -1; h the slot, or the empty slot where an insert
+    // goes; k = {key, epoch, enter, birth} and d the distance (DBL_MAX if absent).
+    __device__ __forceinline__ int vlook(int v, uint32_t& h, int4& k, double& d) const {
+        if constexpr (kCoop) {
+            const ProbeR r = probe1(VT(), C.vcap_log2, (uint32_t)v);
+            h = (uint32_t)(r.slot >= 0 ? r.slot : r.empty);  // vlimit keeps a quarter of the slots empty: never -1
+            k = r.head;
+            d = r.slot >= 0 ? __hiloint2double(r.tail.y, r.tail.x) : DBL_MAX;
+            return r.slot;
+        } else {
+            vfirst(v, h, k, d);
+            return vfinish(v, h, k, d);
+        }
+    }
+    __device__ __forceinline__ int vfind(int v) const {
+        uint32_t h;
+        int4 k;
+        double d;
+        return vlook(v, h, k, d);
+    }
+    __device__ __forceinline__ double vdist(int v) const {
+        uint32_t h;
+        int4 k;
+        double d;
+        vlook(v, h, k, d);
+        return d;
+    }
     __device__ __forceinline__ void sfirst(int e, uint32_t& h, int4& k, double2& dx) const {
         h = shash((uint32_t)e);
         k = *reinterpret_cast<const int4*>(&ST()[h]);
@@ -509,35 +501,17 @@ struct LaneT {
             dx = *reinterpret_cast<const double2*>(&ST()[h].dist);
         }
     }
-    __device__ __forceinline__ double vdist(int v) {
-        int s = vfind(v);
-        return s < 0 ? DBL_MAX : VT()[s].dist;
-    }
-    __device__ __forceinline__ int vbirth(int v) {
-        int s = vfind(v);
-        return s < 0 ? -1 : VT()[s].birth;
-    }
-    // MyHashTable::operator[] (MyHashTable.cuh:72-82): find or insert with defaults
-    __device__ int vput(int v) {
+    __device__ __forceinline__ int sfind(int e) const {
+        if constexpr (kCoop) return probe1(ST(), C.scap_log2, (uint32_t)e).slot;
         uint32_t h;
-        if constexpr (kCoop) {
-            const ProbeR r = probe1(VT(), C.vcap_log2, (uint32_t)v);
-            if (r.slot >= 0) return r.slot;
-            h = (uint32_t)r.empty;  // vlimit keeps a quarter of the slots empty: never -1
-        } else {
-            uint32_t mask = (1u << C.vcap_log2) - 1;
-            h = vhash((uint32_t)v);
-            for (;;) {
-                uint2 ke = *reinterpret_cast<const uint2*>(&VT()[h]);
-                if (ke.y != epoch) break;
-                if (ke.x == (uint32_t)v) return (int)h;
-                h = (h + 1) & mask;
-            }
-        }
-        return vinsert(v, h);
+        int4 k;
+        double2 dx;
+        sfirst(e, h, k, dx);
+        return sfinish(e, h, k, dx);
     }
-    // Insert vertex v at h, the empty slot that ends its probe chain.
-    __device__ int vinsert(int v, uint32_t h) {
+    // Insert vertex v at h, the empty slot that ends its probe chain
+    // (MyHashTable::operator[], MyHashTable.cuh:72-82, with its defaults).
+    __device__ __forceinline__ int vinsert(int v, uint32_t h) {
         if (vcount >= C.vlimit) {  // keep the probe chains short: hand the source to the big pass
             flags |= kFlagCapacity;
             return -1;
@@ -550,36 +524,8 @@ struct LaneT {
         if ((uint32_t)vcount > C.vref) flags |= kFlagRefOverflow;
         return (int)h;
     }
-    __device__ __forceinline__ int sfind(int e) {
-        if constexpr (kCoop) return probe1(ST(), C.scap_log2, (uint32_t)e).slot;
-        uint32_t mask = (1u << C.scap_log2) - 1, h = shash((uint32_t)e);
-        for (;;) {
-            uint2 ke = *reinterpret_cast<const uint2*>(&ST()[h]);
-            if (ke.y != epoch) return -1;
-            if (ke.x == (uint32_t)e) return (int)h;
-            h = (h + 1) & mask;
-        }
-    }
-    __device__ int sput(int e) {
-        uint32_t h;
-        if constexpr (kCoop) {
-            const ProbeR r = probe1(ST(), C.scap_log2, (uint32_t)e);
-            if (r.slot >= 0) return r.slot;
-            h = (uint32_t)r.empty;  // slimit keeps a quarter of the slots empty: never -1
-        } else {
-            uint32_t mask = (1u << C.scap_log2) - 1;
-            h = shash((uint32_t)e);
-            for (;;) {
-                uint2 ke = *reinterpret_cast<const uint2*>(&ST()[h]);
-                if (ke.y != epoch) break;
-                if (ke.x == (uint32_t)e) return (int)h;
-                h = (h + 1) & mask;
-            }
-        }
-        return sinsert(e, h);
-    }
     // Insert half-edge e at h, the empty slot that ends its probe chain.
-    __device__ int sinsert(int e, uint32_t h) {
+    __device__ __forceinline__ int sinsert(int e, uint32_t h) {
         if (scount >= C.slimit) {
             flags |= kFlagCapacity;
             return -1;
@@ -609,20 +555,18 @@ struct LaneT {
     // The reference's sift-up (PriorityQueue.cuh:57-64): the new entry moves up
     // while its parent's key is greater.  On the benchmark mesh 69 % of the
     // window pushes do not move and 11.6 % climb past four levels.  Four
-    // ancestors are loaded per round trip (they are what the level-by-level
-    // loop would read: a move only writes below the next ancestor); the number
-    // of moves over them is counted with the same stop rule and the moves are
-    // written predicated, so no data-dependent branch splits the lanes; with
-    // SVG_UP_BATCHES a longer climb takes the next four the same way, else it
-    // continues level by level.
-    template <class T>
-    __device__ __forceinline__ int sift_up(T* H, int cur, const T& x) {
+    // ancestors' keys are loaded per round trip for as long as the climb goes
+    // on (they are what the level-by-level loop would read: a move only writes
+    // below the next ancestor); the number of moves over them is counted with
+    // the same stop rule and the moves are written predicated, so no
+    // data-dependent branch splits the lanes.
+    __device__ __forceinline__ void sift_up(HeapEntry* H, int cur, const HeapEntry& x) {
         if constexpr (kCoop) {
             // thread j holds ancestor cur >> (j + 1); the moves are the
             // ancestors, from the parent up, whose key exceeds x's
             const int lane = threadIdx.x & 31;
             const int a = lane < 30 ? (cur >> (lane + 1)) : 0;
-            T e;
+            HeapEntry e;
             e.key = 0.0;
             if (a > 0) e = H[a];
             const unsigned gt = __ballot_sync(0xFFFFFFFFu, a > 0 && e.key > x.key);
@@ -630,14 +574,8 @@ struct LaneT {
             if (lane < m) H[cur >> lane] = e;
             H[cur >> m] = x;
             __syncwarp();
-            return cur >> m;
         } else {
-            constexpr int kUp = SVG_KEYS_ONLY_SIFT ? SVG_UP_LEVELS : 4;
-#if SVG_KEYS_ONLY_SIFT && SVG_UP_BATCHES
-            // batches of kUp ancestors' keys, one round trip each, for as long
-            // as the climb goes on: the same stop rule level by level, since a
-            // batch's moves only shift entries below its top ancestor (a
-            // tenth of the pushes climb past four levels)
+            constexpr int kUp = 4;
             int c = cur;
             for (;;) {
                 double ak[kUp];
@@ -647,83 +585,22 @@ struct LaneT {
 #pragma unroll
                 for (int j = 0; j < kUp; ++j)
                     if (m == j && (c >> (j + 1)) > 0 && ak[j] > x.key) m = j + 1;
-                if constexpr (kUp <= SVG_UP_ARRAY) {
-                    T mv[kUp];
+                HeapEntry mv[kUp];
 #pragma unroll
-                    for (int j = 0; j < kUp; ++j)
-                        if (j < m) mv[j] = H[c >> (j + 1)];
+                for (int j = 0; j < kUp; ++j)
+                    if (j < m) mv[j] = H[c >> (j + 1)];
 #pragma unroll
-                    for (int j = 0; j < kUp; ++j)
-                        if (j < m) H[c >> j] = mv[j];
-                } else {
-                    for (int j = 0; j < m; ++j) H[c >> j] = H[c >> (j + 1)];
-                }
+                for (int j = 0; j < kUp; ++j)
+                    if (j < m) H[c >> j] = mv[j];
                 c >>= m;
                 if (m < kUp) break;
             }
             H[c] = x;
-            return c;
-#elif SVG_KEYS_ONLY_SIFT
-            // keys of the first kUp ancestors in one round trip; the moved
-            // entries are read again (their sectors were just fetched) before
-            // each is written one level down
-            double ak[kUp];
-#pragma unroll
-            for (int j = 0; j < kUp; ++j) ak[j] = (cur >> (j + 1)) > 0 ? H[cur >> (j + 1)].key : 0.0;
-            int m = 0;
-#pragma unroll
-            for (int j = 0; j < kUp; ++j)
-                if (m == j && (cur >> (j + 1)) > 0 && ak[j] > x.key) m = j + 1;
-            if constexpr (kUp <= SVG_UP_ARRAY) {
-                T mv[kUp];
-#pragma unroll
-                for (int j = 0; j < kUp; ++j)
-                    if (j < m) mv[j] = H[cur >> (j + 1)];
-#pragma unroll
-                for (int j = 0; j < kUp; ++j)
-                    if (j < m) H[cur >> j] = mv[j];
-            } else {
-                // one entry at a time, top-down reads after the writes below
-                // them (each read hits the sector just fetched)
-                for (int j = 0; j < m; ++j) H[cur >> j] = H[cur >> (j + 1)];
-            }
-#else
-            // the first four ancestors in one round trip (they are what the level-
-            // by-level loop would read: a move only writes below the next
-            // ancestor); the moves over them are counted with the same stop rule
-            // and written predicated
-            T anc[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if ((cur >> (j + 1)) > 0) anc[j] = H[cur >> (j + 1)];
-            int m = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (m == j && (cur >> (j + 1)) > 0 && anc[j].key > x.key) m = j + 1;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < m) H[cur >> j] = anc[j];
-#endif
-#if !(SVG_KEYS_ONLY_SIFT && SVG_UP_BATCHES)
-            int c = cur >> m;
-            if (m == kUp) {
-                for (;;) {
-                    const int p = c >> 1;
-                    if (p == 0) break;
-                    const T pe = H[p];
-                    if (!(pe.key > x.key)) break;
-                    H[c] = pe;
-                    c = p;
-                }
-            }
-            H[c] = x;
-            return c;
-#endif
         }
     }
 
     // Push (PriorityQueue.cuh:48-67).
-    __device__ void wpush(const NewWin& w, int psrc, int birth) {
+    __device__ __forceinline__ void wpush(const NewWin& w, int psrc, int birth) {
         ++st_generated();  // counts attempts, like numOfWinGen
         if (wsize >= C.wcap) {  // PriorityQueue.cuh:53: dropped when full
             flags |= kFlagQueueDrop;
@@ -733,7 +610,6 @@ struct LaneT {
             flags |= kFlagCapacity;
             return;
         }
-#if SVG_FREE_CACHE
         // the list entry under the cached top is loaded now and used by the
         // next push, after this push's sift-up
         int slot;
@@ -743,14 +619,11 @@ struct LaneT {
         } else {
             slot = nfresh++;
         }
-#else
-        const int slot = nfree > 0 ? (int)WF()[--nfree] : nfresh++;
-#endif
         WP()[slot] = w.p;
-        WinEntry e;
+        HeapEntry e;
         e.key = w.key;
-        e.psrc = psrc;
-        e.sb = (uint32_t)slot | ((uint32_t)(birth & 0xFF) << 16);
+        e.id = psrc;
+        e.bits = (uint32_t)slot | ((uint32_t)(birth & 0xFF) << 16);
         sift_up(WH(), ++wsize, e);
         if (wsize > st_maxw()) st_maxw() = wsize;
     }
@@ -760,14 +633,13 @@ struct LaneT {
     // rules below, and each moved node is written by the thread holding it.
     // Every node is read before any write of that round, and a round writes
     // only nodes above the next round's subtree.
-    template <class T>
-    __device__ __forceinline__ int coop_sift_down(T* H, int n, const T& last) {
+    __device__ __forceinline__ int coop_sift_down(HeapEntry* H, int n, const HeapEntry& last) {
         constexpr unsigned kFull = 0xFFFFFFFFu;
         const int lane = threadIdx.x & 31;
         int cur = 1;
         for (int round = 0; round < 8; ++round) {
             if ((cur << 1) > n) break;
-            T e[2];
+            HeapEntry e[2];
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int k = lane + 32 * r;       // subtree node in level order
@@ -801,23 +673,18 @@ struct LaneT {
     // The reference's sift-down (PriorityQueue.cuh:76-105): the children of
     // `cur` are compared with each other (ties go right) and the smaller moves
     // up while it is smaller than the last element.  The keys of three levels
-    // below `cur` (SVG_SIFT3; two without it) are loaded together, so those
-    // levels cost one dependent round trip (reads past the heap's end stay
+    // below `cur` (2 + 4 + 8) are loaded together, so those levels cost one
+    // dependent round trip (two levels a trip measured 2.6 % slower on the
+    // 72.9K height field at K = 500, four 14 %; reads past the heap's end stay
     // inside the lane's array, stride >= cap + 8, and are never used); the
     // moved entries are read again from the sectors just fetched and written
     // with predicated stores, one exit test per round trip.
-    template <class T>
-    __device__ __forceinline__ int sift_down2(T* H, int n, const T& last) {
+    __device__ __forceinline__ int sift_down(HeapEntry* H, int n, const HeapEntry& last) {
         if constexpr (kCoop) return coop_sift_down(H, n, last);
         int cur = 1;
         for (;;) {
             const int l = cur << 1;
             if (l > n) break;
-#if SVG_SIFT3
-            // keys of three levels below cur (2 + 4 + 8) in one round trip
-            // (reads past the heap's end stay inside the lane's array,
-            // stride >= cap + 8, and are never used); the moved entries are
-            // read again from the sectors just fetched
             const double a = H[l].key, b = H[l + 1].key;
             const int g = cur << 2, h8 = cur << 3;
             double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0;
@@ -841,7 +708,7 @@ struct LaneT {
             const int k3 = (l3 + 1 <= n && !(a3 < b3)) ? 1 : 0;
             const bool mv3 = mv2 && l3 <= n && (k3 ? b3 : a3) < last.key;
             const int c3 = l3 + k3;
-            T e1, e2, e3;
+            HeapEntry e1, e2, e3;
             if (mv1) e1 = H[c1];
             if (mv2) e2 = H[c2];
             if (mv3) e3 = H[c3];
@@ -849,62 +716,11 @@ struct LaneT {
             if (mv2) H[c1] = e2;
             if (mv3) H[c2] = e3;
             cur = mv3 ? c3 : (mv2 ? c2 : (mv1 ? c1 : cur));
-            const bool more = mv3;
-#elif SVG_KEYS_ONLY_SIFT
-            const double a = H[l].key, b = H[l + 1].key;
-            const int g = cur << 2;
-            double q0 = 0.0, q1 = 0.0, q2 = 0.0, q3 = 0.0;
-            if (g <= n) { q0 = H[g].key; q1 = H[g + 1].key; q2 = H[g + 2].key; q3 = H[g + 3].key; }
-            const int k1 = (l + 1 <= n && !(a < b)) ? 1 : 0;
-            const bool mv1 = (k1 ? b : a) < last.key;
-            const int c1 = l + k1;
-            const int l2 = c1 << 1;
-            const double a2 = k1 ? q2 : q0, b2 = k1 ? q3 : q1;
-            const int k2 = (l2 + 1 <= n && !(a2 < b2)) ? 1 : 0;
-            const bool mv2 = mv1 && l2 <= n && (k2 ? b2 : a2) < last.key;
-            const int c2 = l2 + k2;
-            T e1, e2;
-            if (mv1) e1 = H[c1];
-            if (mv2) e2 = H[c2];
-            if (mv1) H[cur] = e1;
-            if (mv2) H[c1] = e2;
-            cur = mv2 ? c2 : (mv1 ? c1 : cur);
-            const bool more = mv2;
-#else
-            const T a = H[l], b = H[l + 1];
-            const int g = cur << 2;
-            T q0, q1, q2, q3;
-            if (g <= n) { q0 = H[g]; q1 = H[g + 1]; q2 = H[g + 2]; q3 = H[g + 3]; }
-            const int k1 = (l + 1 <= n && !(a.key < b.key)) ? 1 : 0;
-            const T e1 = k1 ? b : a;
-            const bool mv1 = e1.key < last.key;
-            const int c1 = l + k1;
-            const int l2 = c1 << 1;
-            const T a2 = k1 ? q2 : q0, b2 = k1 ? q3 : q1;
-            const int k2 = (l2 + 1 <= n && !(a2.key < b2.key)) ? 1 : 0;
-            const T e2 = k2 ? b2 : a2;
-            const bool mv2 = mv1 && l2 <= n && e2.key < last.key;
-            if (mv1) H[cur] = e1;
-            if (mv2) H[c1] = e2;
-            cur = mv2 ? l2 + k2 : (mv1 ? c1 : cur);
-            const bool more = mv2;
-#endif
-            if (!more) break;
+            if (!mv3) break;
         }
         return cur;
     }
-    __device__ WinEntry wpop() {
-        const WinEntry top = WH()[1];
-        WinEntry last = WH()[wsize];
-        const int n = --wsize;
-        const int cur = sift_down2(WH(), n, last);
-        WH()[cur] = last;
-        WF()[nfree++] = (uint16_t)(top.sb & 0xFFFF);
-        ftop = (int)(top.sb & 0xFFFF);
-        if constexpr (kCoop) __syncwarp();
-        return top;
-    }
-    __device__ void ppush(double key, int vert, int level, int birth) {
+    __device__ __forceinline__ void ppush(double key, int vert, int level, int birth) {
         if (psize >= C.pcap) {
             flags |= kFlagQueueDrop;
             return;
@@ -913,31 +729,23 @@ struct LaneT {
             flags |= kFlagCapacity;
             return;
         }
-        PsEntry e;
-        e.key = key; e.vert = vert; e.lb = ((uint32_t)level << 8) | (uint32_t)(birth & 0xFF);
+        HeapEntry e;
+        e.key = key; e.id = vert; e.bits = ((uint32_t)level << 8) | (uint32_t)(birth & 0xFF);
         if constexpr (kCoop) {
             sift_up(PH(), ++psize, e);
         } else {
+            HeapEntry* H = PH();
             int cur = ++psize, p = cur >> 1;
             while (p > 0) {
-                PsEntry pe = ph(p);
+                const HeapEntry pe = H[p];
                 if (!(pe.key > key)) break;
-                ph(cur) = pe;
+                H[cur] = pe;
                 cur = p;
                 p = cur >> 1;
             }
-            ph(cur) = e;
+            H[cur] = e;
         }
         if (psize > st_maxp()) st_maxp() = psize;
-    }
-    __device__ PsEntry ppop() {
-        const PsEntry top = PH()[1];
-        PsEntry last = PH()[psize];
-        const int n = --psize;
-        const int cur = sift_down2(PH(), n, last);
-        PH()[cur] = last;
-        if constexpr (kCoop) __syncwarp();
-        return top;
     }
 
     // -------------------------------------------------- source lifecycle
@@ -952,7 +760,6 @@ struct LaneT {
         st_steps() = 0;
         src_birth = 0;
         done = false;
-        pk_valid = false;
         if (clear_all) {
             clear_tables();  // every slot now carries epoch 0 = empty
             epoch = 1;
@@ -960,7 +767,13 @@ struct LaneT {
             ++epoch;
             if (epoch == 0) ++epoch;
         }
-        initialize();
+        // ICHDevice::Initialize (ICHDevice.cu:525-581) is the fan of the source
+        // itself: the lane's first action, run with the pseudo-sources' fans
+        pk_valid = true;
+        pk_act = kActPseudo;
+        pk_proc = true;
+        pk_init = true;
+        set_pending(0.0, v, 0u);
     }
     __device__ void save_epoch(int gtid) { C.epochs[gtid] = epoch; }
 
@@ -970,263 +783,132 @@ struct LaneT {
         if (v == source) src_birth = b;
     }
 
-    // ICHDevice::Initialize, vertex source (ICHDevice.cu:525-581)
-    __device__ void initialize() {
-        const DevMesh& M = C.M;
-        int start = __ldg(&M.vr[source].first);
-        if (start < 0) {  // isolated vertex: the reference indexes edges[-1]
-            flags |= kFlagUndefined;
-            return;
-        }
-        int cur = start;
-        int guard = 0;
-        do {
-            if (++guard > 1 << 20) { flags |= kFlagWatchdog; return; }
-            HeRec hc = ld_he(M.he, cur);
-            int op = nxt(cur);
-            HeRec ho = ld_he(M.he, op);
-            HeRec hp = ld_he(M.he, prv(cur));
-            NewWin w;
-            finish_window(0.0, ho.len, hc.len, hp.len, 0.0, w);
-            w.p.cross = ho.twin;
-            w.p.level = 0;
-            wpush(w, source, 0);
-            int opv = hc.v1;
-            int s = vput(opv);
-            if (s < 0) return;
-            if (hc.len > VT()[s].dist) {
-                cur = hc.twin;
-                if (cur != -1) cur = nxt(cur);
-                continue;
-            }
-            set_birth(s, opv, 0);
-            VT()[s].dist = hc.len;
-            VT()[s].enter = hc.twin;
-            VT()[s].sslot = -1;
-            if (!(__ldg(&M.vr[opv].flags) & kVertSaddleGE)) {
-                cur = hc.twin;
-                if (cur != -1) cur = nxt(cur);
-                continue;
-            }
-            ppush(hc.len, opv, 0, VT()[s].birth);
-            cur = hc.twin;
-            if (cur != -1) cur = nxt(cur);
-        } while (cur != start && cur != -1);
-        int s = vput(source);
-        if (s < 0) return;
-        set_birth(s, source, 0);
-        VT()[s].dist = 0.0;
-        VT()[s].enter = -1;
-        VT()[s].sslot = -1;
-    }
-
     // ICHDevice::IsValidWindow (ICHDevice.cu:906-955) given the distances d1,
     // d2, d3 of the window half-edge's start, end and opposite vertex; l0 its
     // length; (tx,ty) the opposite vertex in the window's frame.
     __device__ __forceinline__ bool valid_window(const NewWin& w, bool isLeft, double d1, double d2, double d3,
                                                  double l0, double tx, double ty) const {
         const WinPay& p = w.p;
-        if (p.b1 <= p.b0) return false;
         const double dB = hyp(p.sx - p.b1, p.sy - 0.0);
         const double dA = hyp(p.sx - p.b0, p.sy - 0.0);
-        if (p.psd + dB > d1 + p.b1 && (p.psd + dB) / (d1 + p.b1) - 1.0 > 0.0) return false;
-        if (p.psd + dA > d2 + l0 - p.b0 && (p.psd + dA) / (d2 + l0 - p.b0) - 1.0 > 0.0) return false;
         const double q = isLeft ? hyp(tx - p.b0, ty - 0.0) : hyp(tx - p.b1, ty - 0.0);
-        const double dd = isLeft ? dA : dB;
-        const double thr = isLeft ? 0.0 : kRelErr;
-        if (p.psd + dd > d3 + q && (p.psd + dd) / (d3 + q) - 1.0 > thr) return false;
-        return true;
+        const double a = p.psd + (isLeft ? dA : dB), b = d3 + q;
+        return !(p.b1 <= p.b0) && !exceeds(p.psd + dB, d1 + p.b1) && !exceeds(p.psd + dA, d2 + l0 - p.b0) &&
+               !(a > b && (isLeft ? b >= 0.0 : exceeds_rel(a, b)));
     }
 
-    // ICHDevice::BuildWindow (ICHDevice.cu:957-973); (v0x,v0y)-(v1x,v1y) is the
-    // child's half-edge in the parent's frame, cross the twin of that half-edge.
-    __device__ __forceinline__ void build_window(const WinPay& f, int cross, double elen, double t0, double t1,
-                                                 double v0x, double v0y, double v1x, double v1y, NewWin& w) {
-        double b0 = (1 - t0) * elen, b1 = (1 - t1) * elen;
-        double px = v0x * t0 + v1x * (1 - t0), py = v0y * t0 + v1y * (1 - t0);
-        double d0 = hyp(f.sx - px, f.sy - py);
-        px = v0x * t1 + v1x * (1 - t1);
-        py = v0y * t1 + v1y * (1 - t1);
-        double d1 = hyp(f.sx - px, f.sy - py);
-        finish_window(b0, b1, d0, d1, f.psd, w);
-        w.p.cross = cross;
-        w.p.level = f.level + 1;
-    }
+    // ------------------------------------------------------------- actions
+    // One iteration of ICHDevice::Execute's loop (ICHDevice.cu:72-119), split
+    // into take() - which entry comes off next, and its pop - and act() - its
+    // processing.  The reference first pops every outdated window, then every
+    // outdated pseudo-source (birth time no longer that of its pseudo-source
+    // vertex, :80-86), then processes the smaller top; here one outdated entry
+    // is popped per look, in the same order, which removes the same entries
+    // (those pops change nothing else), and a processing action follows once
+    // both tops are current.
+    //   kActWindow  a window (processed: PropagateWindow, ICHDevice.cu:618-726)
+    //   kActPseudo  a pseudo-source (processed: GenSubWinsForPseudoSrc, :728-793)
+    //   kActDone    the source is finished
+    // The popped entry waits in shared memory until act() runs, so a lane may
+    // wait for its warp's vote; nothing touches its heaps meanwhile.
+    enum { kActWindow = 0, kActPseudo = 1, kActDone = 2 };
 
-    // ICHDevice::PropagateWindow (ICHDevice.cu:618-726).  The face beyond the
-    // window is e0 -> e1 -> e2 (e0 = twin of the window's half-edge) with
-    // vertices A = v0(e0), B = v1(e0) and the opposite vertex C = v1(e1).  The
-    // child on e1 (B->C) tests its validity against B, C, A and the child on
-    // e2 (C->A) against C, A, B, so the three distances are probed once, in
-    // parallel with the split entry of e0, and both children are built by one
-    // code path: child 0 = left (frame (0,0)->apex), child 1 = right (frame
-    // apex->(l0,0)).
-    // All lanes of `amask` call this together and meet at each __syncwarp, so
-    // the phases run converged; a lane with nothing to do (live == false, or a
-    // boundary edge, or a full table) only predicates its work off.
-    __device__ void propagate(const WinPay& win, int psrc, int birth, bool live, unsigned amask) {
-        const DevMesh& M = C.M;
-        const int e0 = win.cross;
-        live = live && e0 != -1;
-        int e1 = 0, e2 = 0, A = 0, B = 0, Cv = 0;
-        HeRec h0, h1, h2;
-        double2 v2 = make_double2(0.0, 0.0), top1 = v2, top2 = v2;
-        uint32_t hA = 0, hB = 0, hC = 0, hS = 0;
-        int4 kA = make_int4(0, 0, 0, 0), kB = kA, kC = kA, kS = kA;
-        double dA = 0.0, dB = 0.0, dC = 0.0;
-        double2 sdx = v2;
-        int sC = -1, sS = -1;
-        if (live) {
-            e1 = nxt(e0);
-            e2 = nxt(e1);
-            h0 = ld_he(M.he, e0);
-            h1 = ld_he(M.he, e1);
-            h2 = ld_he(M.he, e2);
-            v2 = ld_apex(M.geo, e0);
-            top1 = ld_top(M.geo, e1);
-            top2 = ld_top(M.geo, e2);
-            A = h0.v0;
-            B = h0.v1;
-            Cv = h1.v1;
-            if constexpr (!kCoop) {
-                vfirst(A, hA, kA, dA);
-                vfirst(B, hB, kB, dB);
-                vfirst(Cv, hC, kC, dC);
-                sfirst(e0, hS, kS, sdx);
-                vfinish(A, hA, kA, dA);
-                vfinish(B, hB, kB, dB);
-                sC = vfinish(Cv, hC, kC, dC);
-                sS = sfinish(e0, hS, kS, sdx);
+    // Up to kInlineStale outdated entries are dropped on the way to a current
+    // one instead of spending a voted action each.  Every pop of the lane -
+    // window or pseudo-source, outdated or current - is the one copy of the
+    // sift-down below: the loop's code decides its instruction-cache misses.
+    template <int kInlineStale>
+    __device__ __forceinline__ int take() {
+        if (pk_valid) return pk_act;
+        pk_valid = true;
+        pk_init = false;
+        for (int inl = 0;; ++inl) {
+            HeapEntry t;
+            const int a = look(t);
+            pk_act = a;
+            if (a == kActDone) return a;
+            const bool w = a == kActWindow;
+            if (w && pk_proc) {  // the payload travels while the sift-down runs
+                const WinPay* p = WP() + (t.bits & 0xFFFF);
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    copy_async16(&g_lane_smem.pay[k][threadIdx.x], reinterpret_cast<const int4*>(p) + k);
             }
-        }
-        if constexpr (kCoop) {  // the four lookups in one group probe (live is the same in every thread)
-            ProbeR ra, rb, rc, rs;
-            coop_probe4(probe_q(VT(), C.vcap_log2, (uint32_t)A, live), probe_q(VT(), C.vcap_log2, (uint32_t)B, live),
-                        probe_q(VT(), C.vcap_log2, (uint32_t)Cv, live), probe_q(ST(), C.scap_log2, (uint32_t)e0, live),
-                        epoch, ra, rb, rc, rs);
-            dA = ra.slot >= 0 ? __hiloint2double(ra.tail.y, ra.tail.x) : DBL_MAX;
-            dB = rb.slot >= 0 ? __hiloint2double(rb.tail.y, rb.tail.x) : DBL_MAX;
-            dC = rc.slot >= 0 ? __hiloint2double(rc.tail.y, rc.tail.x) : DBL_MAX;
-            sC = rc.slot;
-            kC = rc.head;
-            sS = rs.slot;
-            sdx = rs.slot >= 0 ? make_double2(__hiloint2double(rs.tail.y, rs.tail.x),
-                                              __hiloint2double(rs.tail.w, rs.tail.z))
-                               : make_double2(DBL_MAX, DBL_MAX);
-        }
-        __syncwarp(amask);
-
-        const double sx = win.sx, sy = win.sy;
-        const double l0 = h0.len;
-        bool keep0 = live, keep1 = live, both = false;
-        double interX = 0.0;
-        if (live) {
-            interX = v2.x - v2.y * (v2.x - sx) / (v2.y - sy);
-            if (interX <= win.b0) {
-                keep0 = false;  // right child only
-            } else if (interX >= win.b1) {
-                keep1 = false;  // left child only
+            HeapEntry* H = w ? WH() : PH();
+            int n = w ? wsize : psize;
+            const HeapEntry last = H[n];
+            --n;
+            H[sift_down(H, n, last)] = last;
+            if constexpr (kCoop) __syncwarp();
+            if (w) {
+                wsize = n;
+                ftop = (int)(t.bits & 0xFFFF);
+                WF()[nfree++] = (uint16_t)ftop;
             } else {
-                both = true;
-                const double D = hyp(v2.x - sx, v2.y - sy) + win.psd;
-                const double sd = sdx.x;
-                if (D > sd && D / sd - 1.0 > kRelErr) {  // one angle, one split
-                    keep0 = sdx.y < interX;
-                    keep1 = !keep0;
-                } else {
-                    int ssl = sS;
-                    bool ok = true;
-                    if (D < sd) {
-#if SVG_INSERT_AT
-                        // the lookup's chain ended at the empty slot (hS)
-                        ssl = sS >= 0 ? sS : (kCoop ? sput(e0) : sinsert(e0, hS));
-#else
-                        ssl = sS >= 0 ? sS : sput(e0);
-#endif
-                        if (ssl < 0) {
-                            ok = false;  // table full: the source goes to the retry pass
-                        } else {
-                            ST()[ssl].dist = D;
-                            ST()[ssl].psrc = psrc;
-                            ST()[ssl].x = l0 - interX;
-                        }
-                    }
-                    if (ok && D < dC) {
-                        if (dC == DBL_MAX) ++total;
-#if SVG_INSERT_AT
-                        const int s = sC >= 0 ? sC : (kCoop ? vput(Cv) : vinsert(Cv, hC));
-#else
-                        const int s = sC >= 0 ? sC : vput(Cv);
-#endif
-                        if (s < 0) {
-                            ok = false;
-                        } else {
-                            const int b = (int)(signed char)((sC >= 0 ? kC.w : -1) + 1);
-                            set_birth(s, Cv, b);
-                            VT()[s].dist = D;
-                            VT()[s].enter = e0;
-                            VT()[s].sslot = ssl;  // D < dC <= split distance: the entry was just written
-                            dC = D;  // the children's tests read the updated distance
-                            if (__ldg(&M.vr[Cv].flags) & kVertSaddleGT) ppush(D, Cv, win.level + 1, b);
-                        }
-                    }
-                    if (!ok) keep0 = keep1 = false;
-                }
+                psize = n;
+            }
+            if (pk_proc || inl >= kInlineStale) {
+                set_pending(t.key, t.id, t.bits);
+                return a;
             }
         }
-        __syncwarp(amask);
+    }
 
-#if SVG_SEQ_CHILD
-        // One child at a time through one copy of the code: build, test,
-        // push.  The tests read only the three distances, which a push does
-        // not change, so the heap sees the pushes in the same order.
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-            const bool left = c == 0;
-            bool keep = left ? keep0 : keep1;
-            NewWin W;
-            if (keep) {
-                // child 0: frame (0,0) -> apex; child 1: apex -> (l0,0)
-                const double f0x = left ? 0.0 : v2.x, f0y = left ? 0.0 : v2.y;
-                const double f1x = left ? v2.x : l0, f1y = left ? v2.y : 0.0;
-                const bool fix0 = !left && both, fix1 = left && both;
-                const double t0 = fix0 ? 1.0 : isect(sx, sy, win.b0, 0.0, f0x, f0y, f1x, f1y);
-                const double t1 = fix1 ? 0.0 : isect(sx, sy, win.b1, 0.0, f0x, f0y, f1x, f1y);
-                const double elen = left ? h1.len : h2.len;
-                build_window(win, left ? h1.twin : h2.twin, elen, t0, t1, f0x, f0y, f1x, f1y, W);
-                keep = left ? valid_window(W, true, dB, dC, dA, elen, top1.x, top1.y)
-                            : valid_window(W, false, dC, dA, dB, elen, top2.x, top2.y);
-            }
-            __syncwarp(amask);
-            if (keep) wpush(W, psrc, birth);
-            __syncwarp(amask);
+    // Which heap's top comes off next (t), and whether it is current (pk_proc).
+    __device__ __forceinline__ int look(HeapEntry& t) {
+        pk_proc = false;
+        if (done || (wsize == 0 && psize == 0) || (flags & (kFlagCapacity | kFlagWatchdog | kFlagUndefined))) {
+            done = true;
+            return kActDone;
         }
+        if (++st_steps() > C.watchdog) {
+            flags |= kFlagWatchdog;
+            done = true;
+            return kActDone;
+        }
+        HeapEntry pw, pp;
+        pw.key = 0.0; pw.id = 0; pw.bits = 0;
+        pp.key = 0.0; pp.id = 0; pp.bits = 0;
+        if (wsize > 0) pw = WH()[1];
+        if (psize > 0) pp = PH()[1];
+        // both birth lookups issued together
+        const bool wlook = wsize > 0 && pw.id != source;
+        const bool plook = psize > 0;
+        int wb = src_birth, pb = -1;
+        if constexpr (kCoop) {
+            ProbeR rw, rp, r2, r3;
+            coop_probe4(probe_q(VT(), C.vcap_log2, (uint32_t)pw.id, wlook),
+                        probe_q(VT(), C.vcap_log2, (uint32_t)pp.id, plook), probe_off(), probe_off(), epoch, rw,
+                        rp, r2, r3);
+            if (wlook) wb = rw.slot < 0 ? -1 : rw.head.w;
+            if (plook) pb = rp.slot < 0 ? -1 : rp.head.w;
+        } else {
+            uint32_t hw = 0, hp = 0;
+            int4 kw = make_int4(0, 0, 0, 0), kp = make_int4(0, 0, 0, 0);
+            double dw = 0.0, dp = 0.0;
+            if (wlook) vfirst(pw.id, hw, kw, dw);
+            if (plook) vfirst(pp.id, hp, kp, dp);
+            if (wlook) wb = vfinish(pw.id, hw, kw, dw) < 0 ? -1 : kw.w;
+            if (plook) pb = vfinish(pp.id, hp, kp, dp) < 0 ? -1 : kp.w;
+        }
+        t = pw;
+        if (wsize > 0 && (int)(signed char)(pw.bits >> 16) != wb) return kActWindow;
+        if (psize > 0 && (int)(signed char)(pp.bits & 0xFF) != pb) {
+            t = pp;
+            return kActPseudo;
+        }
+        pk_proc = true;
+        if (wsize > 0 && (psize == 0 || pw.key < pp.key)) return kActWindow;
+        t = pp;
+        if (psize > 0 && (wsize == 0 || pw.key >= pp.key)) return kActPseudo;
+        flags |= kFlagWatchdog;  // NaN keys: neither branch is taken; the reference spins
+        done = true;
+        return kActDone;
     }
-#else
-        NewWin W0, W1;
-        if (keep0) {
-            const double t0 = isect(sx, sy, win.b0, 0.0, 0.0, 0.0, v2.x, v2.y);
-            const double t1 = both ? 0.0 : isect(sx, sy, win.b1, 0.0, 0.0, 0.0, v2.x, v2.y);
-            build_window(win, h1.twin, h1.len, t0, t1, 0.0, 0.0, v2.x, v2.y, W0);
-            keep0 = valid_window(W0, true, dB, dC, dA, h1.len, top1.x, top1.y);
-        }
-        if (keep1) {
-            const double t0 = both ? 1.0 : isect(sx, sy, win.b0, 0.0, v2.x, v2.y, l0, 0.0);
-            const double t1 = isect(sx, sy, win.b1, 0.0, v2.x, v2.y, l0, 0.0);
-            build_window(win, h2.twin, h2.len, t0, t1, v2.x, v2.y, l0, 0.0, W1);
-            keep1 = valid_window(W1, false, dC, dA, dB, h2.len, top2.x, top2.y);
-        }
-        __syncwarp(amask);
-        if (keep0) wpush(W0, psrc, birth);
-        __syncwarp(amask);
-        if (keep1) wpush(W1, psrc, birth);
-        __syncwarp(amask);
-    }
-#endif
 
     // Fan walks of GenSubWinsForPseudoSrcFrom{Window,PseudoSrc}
     // (ICHDevice.cu:821-857, 867-903) with precomputed corner angles.
-    __device__ void fan_walk(int left, int right, double a0, double a1, int& startEdge, int& endEdge) {
+    __device__ __forceinline__ void fan_walk(int left, int right, double a0, double a1, int& startEdge, int& endEdge) {
         const DevMesh& M = C.M;
         startEdge = -1;
         endEdge = -1;
@@ -1249,245 +931,354 @@ struct LaneT {
         if (cur != -1) endEdge = ld_he(M.he, nxt(nxt(ld_he(M.he, cur).twin))).twin;
     }
 
-    // ICHDevice::GenSubWinsForPseudoSrc (ICHDevice.cu:728-793).  Called by
-    // the lanes of `amask` together (see propagate); `live` predicates.
-    __device__ void gen_sub_wins(double pdist, int pv, int plevel, int pbirth, bool live, unsigned amask) {
+    // Where the fan of pseudo-source pv starts and ends
+    // (ICHDevice::GenSubWinsForPseudoSrc, ICHDevice.cu:728-760); false where
+    // the reference leaves it undefined.
+    __device__ __forceinline__ bool fan_range(int pv, int& startEdge, int& endEdge) {
         const DevMesh& M = C.M;
-        int startEdge = -1, endEdge = -1;
-        if (live) {
-            int vs = vfind(pv);
-            int enter = vs < 0 ? -1 : VT()[vs].enter;
-            int vb = vs < 0 ? -1 : VT()[vs].birth;
-            if (enter == -1 && vb != -1) {
-                startEdge = __ldg(&M.vr[pv].first);
-                endEdge = startEdge;
-            } else if (enter >= 0 && ld_he(M.he, enter).v0 == pv) {
-                fan_walk(enter, ld_he(M.he, enter).twin, 0.0, 0.0, startEdge, endEdge);
-            } else if (enter >= 0 && ld_he(M.he, nxt(enter)).v1 == pv) {
-                // GenSubWinsForPseudoSrcFromWindow (ICHDevice.cu:795-858)
-                int e0 = enter, e1 = nxt(e0), e2 = nxt(e1);
-                HeRec h0 = ld_he(M.he, e0), h1 = ld_he(M.he, e1), h2 = ld_he(M.he, e2);
-                double l0 = h0.len, l1 = h1.len, l2 = h2.len;
-                int ss = sfind(e0);
-                double sx = ss < 0 ? DBL_MAX : ST()[ss].x;
-                double ex = l0 - sx, ey = 0.0;
-                double2 v2 = ld_apex(M.geo, e0);
-                double dx = ex - v2.x, dy = ey - v2.y;
-                double dl = hyp(dx, dy);
-                double a0 = (dx * (0.0 - v2.x) + dy * (0.0 - v2.y)) / dl / l1;
-                double a1 = (dx * (l0 - v2.x) + dy * (0.0 - v2.y)) / dl / l2;
-                if (a0 > 1.0) a0 = 1.0; else if (a0 < -1.0) a0 = -1.0;
-                if (a1 > 1.0) a1 = 1.0; else if (a1 < -1.0) a1 = -1.0;
-                a0 = acos(a0);
-                a1 = acos(a1);
-                fan_walk(h1.twin, h2.twin, a0, a1, startEdge, endEdge);
-            } else {
-                flags |= kFlagUndefined;  // assert(false) at ICHDevice.cu:740
-                live = false;
-            }
-            if (flags & kFlagWatchdog) live = false;
+        uint32_t h;
+        int4 k;
+        double d;
+        const int vs = vlook(pv, h, k, d);
+        const int enter = vs < 0 ? -1 : k.z;
+        const int vb = vs < 0 ? -1 : k.w;
+        int left, right;
+        double a0 = 0.0, a1 = 0.0;
+        if (enter == -1 && vb != -1) {
+            startEdge = endEdge = __ldg(&M.vr[pv].first);
+            return true;
         }
-        __syncwarp(amask);
-        if (live) {
-            int guard = 0;
-            do {
-                if (startEdge < 0) {  // the reference reads edges[-1] here
-                    flags |= kFlagUndefined;
-                    break;
-                }
-                int we = nxt(startEdge);
-                HeRec hs = ld_he(M.he, startEdge), hw = ld_he(M.he, we);
-                HeRec hn = ld_he(M.he, nxt(we));
-                NewWin w;
-                finish_window(0.0, hw.len, hs.len, hn.len, pdist, w);
-                w.p.cross = hw.twin;
-                w.p.level = plevel + 1;
-                wpush(w, pv, pbirth);
-                startEdge = hn.twin;
-                if (++guard > 1 << 20) { flags |= kFlagWatchdog; live = false; break; }
-            } while (startEdge != endEdge);
+        if (enter < 0) {
+            flags |= kFlagUndefined;  // assert(false) at ICHDevice.cu:740
+            return false;
         }
-        __syncwarp(amask);
-        if (live) {
-            int start = __ldg(&M.vr[pv].first), cur = start;
-            int guard = 0;
-            do {
-                if (++guard > 1 << 20) { flags |= kFlagWatchdog; break; }
-                HeRec hc = ld_he(M.he, cur);
-                int opv = hc.v1;
-                int os = vfind(opv);
-                double od = os < 0 ? DBL_MAX : VT()[os].dist;
-                if (!(__ldg(&M.vr[opv].flags) & kVertSaddleGE) || od < pdist + hc.len) {
-                    cur = hc.twin;
-                    if (cur != -1) cur = nxt(cur);
-                    continue;
-                }
-                if (od == DBL_MAX) ++total;
-                int s = os < 0 ? vput(opv) : os;
-                if (s < 0) break;
-                VT()[s].dist = pdist + hc.len;
-                int b = (int)(signed char)(VT()[s].birth + 1);
-                set_birth(s, opv, b);
-                VT()[s].enter = hc.twin;
-                VT()[s].sslot = -1;
-                ppush(VT()[s].dist, opv, plevel, b);
-                cur = hc.twin;
-                if (cur != -1) cur = nxt(cur);
-            } while (cur != start && cur != -1);
-        }
-        __syncwarp(amask);
-    }
-
-    // One iteration of ICHDevice::Execute's loop (ICHDevice.cu:72-119),
-    // split into peek() - which entry comes off next - and act() - pop it
-    // and process it.  The reference first pops every outdated window, then
-    // every outdated pseudo-source (birth time no longer that of its
-    // pseudo-source vertex, :80-86), then processes the smaller top; here one
-    // outdated entry is popped per action, in the same order, which removes
-    // the same entries (those pops change nothing else), and a processing
-    // action follows once both tops are current.
-    //   kActWindow  pop the window top (outdated, or processed: PropagateWindow)
-    //   kActPseudo  pop the pseudo-source top (outdated, or GenSubWinsForPseudoSrc)
-    //   kActDone    the source is finished
-    // peek() caches its decision until act() runs, so a lane may wait.
-    enum { kActWindow = 0, kActPseudo = 1, kActDone = 2 };
-    bool done;
-    bool pk_valid;
-    int pk_act;
-    bool pk_proc;  // process (true) or just drop an outdated entry (false)
-#if SVG_SMEM_STATE
-    __device__ __forceinline__ void set_pk(const WinEntry& w, const PsEntry& p) const {
-        const int t = threadIdx.x;
-        g_lane_smem.wkey[t] = w.key; g_lane_smem.wpsrc[t] = w.psrc; g_lane_smem.wsb[t] = w.sb;
-        g_lane_smem.pkey[t] = p.key; g_lane_smem.pvert[t] = p.vert; g_lane_smem.plb[t] = p.lb;
-    }
-    __device__ __forceinline__ WinEntry pk_w() const {
-        const int t = threadIdx.x;
-        WinEntry w;
-        w.key = g_lane_smem.wkey[t]; w.psrc = g_lane_smem.wpsrc[t]; w.sb = g_lane_smem.wsb[t];
-        return w;
-    }
-    __device__ __forceinline__ PsEntry pk_p() const {
-        const int t = threadIdx.x;
-        PsEntry p;
-        p.key = g_lane_smem.pkey[t]; p.vert = g_lane_smem.pvert[t]; p.lb = g_lane_smem.plb[t];
-        return p;
-    }
-#else
-    WinEntry pkw_;
-    PsEntry pkp_;
-    __device__ __forceinline__ void set_pk(const WinEntry& w, const PsEntry& p) { pkw_ = w; pkp_ = p; }
-    __device__ __forceinline__ WinEntry pk_w() const { return pkw_; }
-    __device__ __forceinline__ PsEntry pk_p() const { return pkp_; }
-#endif
-
-    // Up to this many outdated tops (pseudo-source reborn since the entry was
-    // queued) are popped inside peek() instead of spending a voted step each;
-    // the lane's heap operations happen in the same order either way.
-    // The batched kernel passes SVG_ICH_INLINE_STALE; a lane stepping on its
-    // own (the plain form) gains nothing from it and passes 0, which compiles
-    // to a single look at the tops.
-    template <int kInlineStale>
-    __device__ int peek() {
-        if (pk_valid) return pk_act;
-        pk_valid = true;
-        for (int inl = 0;; ++inl) {
-            const int a = peek_once();
-            if (a == kActDone || pk_proc || inl >= kInlineStale) return a;
-            if (a == kActWindow) wpop();   // what act_window does with an outdated top
-            else ppop();                   // likewise act_pseudo
-        }
-    }
-
-    __device__ int peek_once() {
-        pk_proc = false;
-        if (done || (wsize == 0 && psize == 0) || (flags & (kFlagCapacity | kFlagWatchdog | kFlagUndefined))) {
-            done = true;
-            return pk_act = kActDone;
-        }
-        if (++st_steps() > C.watchdog) {
-            flags |= kFlagWatchdog;
-            done = true;
-            return pk_act = kActDone;
-        }
-        WinEntry pw;
-        PsEntry pp;
-        pw.key = 0.0; pw.psrc = 0; pw.sb = 0;
-        pp.key = 0.0; pp.vert = 0; pp.lb = 0;
-        if (wsize > 0) pw = WH()[1];
-        if (psize > 0) pp = PH()[1];
-        set_pk(pw, pp);
-        // both birth lookups issued together
-        const bool wlook = wsize > 0 && pw.psrc != source;
-        const bool plook = psize > 0;
-        int wb = src_birth, pb = -1;
-        if constexpr (kCoop) {
-            ProbeR rw, rp, r2, r3;
-            coop_probe4(probe_q(VT(), C.vcap_log2, (uint32_t)pw.psrc, wlook),
-                        probe_q(VT(), C.vcap_log2, (uint32_t)pp.vert, plook), probe_off(), probe_off(), epoch, rw,
-                        rp, r2, r3);
-            if (wlook) wb = rw.slot < 0 ? -1 : rw.head.w;
-            if (plook) pb = rp.slot < 0 ? -1 : rp.head.w;
+        const int e1 = nxt(enter);
+        const HeRec h0 = ld_he(M.he, enter), h1 = ld_he(M.he, e1);
+        if (h0.v0 == pv) {
+            left = enter;
+            right = h0.twin;
+        } else if (h1.v1 == pv) {
+            // GenSubWinsForPseudoSrcFromWindow (ICHDevice.cu:795-858)
+            const HeRec h2 = ld_he(M.he, nxt(e1));
+            const double l0 = h0.len, l1 = h1.len, l2 = h2.len;
+            int ss = sfind(enter);
+            double sx = ss < 0 ? DBL_MAX : ST()[ss].x;
+            double ex = l0 - sx, ey = 0.0;
+            double2 v2 = ld_apex(M.geo, enter);
+            double dx = ex - v2.x, dy = ey - v2.y;
+            double dl = hyp(dx, dy);
+            a0 = (dx * (0.0 - v2.x) + dy * (0.0 - v2.y)) / dl / l1;
+            a1 = (dx * (l0 - v2.x) + dy * (0.0 - v2.y)) / dl / l2;
+            if (a0 > 1.0) a0 = 1.0; else if (a0 < -1.0) a0 = -1.0;
+            if (a1 > 1.0) a1 = 1.0; else if (a1 < -1.0) a1 = -1.0;
+            a0 = acos(a0);
+            a1 = acos(a1);
+            left = h1.twin;
+            right = h2.twin;
         } else {
-            uint32_t hw = 0, hp = 0;
-            int4 kw = make_int4(0, 0, 0, 0), kp = make_int4(0, 0, 0, 0);
-            double dw = 0.0, dp = 0.0;
-            if (wlook) vfirst(pw.psrc, hw, kw, dw);
-            if (plook) vfirst(pp.vert, hp, kp, dp);
-            if (wlook) wb = vfinish(pw.psrc, hw, kw, dw) < 0 ? -1 : kw.w;
-            if (plook) pb = vfinish(pp.vert, hp, kp, dp) < 0 ? -1 : kp.w;
+            flags |= kFlagUndefined;
+            return false;
         }
-        const bool wstale = wsize > 0 && (int)(signed char)(pw.sb >> 16) != wb;
-        if (wstale) return pk_act = kActWindow;
-        const bool pstale = psize > 0 && (int)(signed char)(pp.lb & 0xFF) != pb;
-        if (pstale) return pk_act = kActPseudo;
-        pk_proc = true;
-        if (wsize > 0 && (psize == 0 || pw.key < pp.key)) return pk_act = kActWindow;
-        if (psize > 0 && (wsize == 0 || pw.key >= pp.key)) return pk_act = kActPseudo;
-        flags |= kFlagWatchdog;  // NaN keys: neither branch is taken; the reference spins
-        done = true;
-        return pk_act = kActDone;
+        fan_walk(left, right, a0, a1, startEdge, endEdge);
+        return !(flags & kFlagWatchdog);
     }
 
-    // Pop the window top; process it if peek() said so.  The lanes of amask
-    // call this together (each of them with its own top).
-    __device__ void act_window(unsigned amask) {
+    // The neighbours of pseudo-source pv (or, init, of the source): distances
+    // along the edges, saddle neighbours queued as pseudo-sources
+    // (ICHDevice.cu:762-792; ICHDevice.cu:549-580 for the source, which also
+    // records neighbours that are no saddles).
+    __device__ __forceinline__ void ring(double pdist, int pv, int level, bool init) {
+        const DevMesh& M = C.M;
+        const int start = __ldg(&M.vr[pv].first);
+        int cur = start;
+        int guard = 0;
+        do {
+            if (++guard > 1 << 20) { flags |= kFlagWatchdog; return; }
+            const HeRec hc = ld_he(M.he, cur);
+            cur = hc.twin;
+            if (cur != -1) cur = nxt(cur);
+            const int opv = hc.v1;
+            if (!init && !(hc.vflags & kVertSaddleGE)) continue;
+            uint32_t h;
+            int4 k;
+            double od;
+            int s = vlook(opv, h, k, od);
+            const double nd = pdist + hc.len;
+            if (od < nd) continue;
+            if (!init && od == DBL_MAX) ++total;
+            int b = init || s < 0 ? 0 : (int)(signed char)(k.w + 1);
+            if (s < 0) s = vinsert(opv, h);
+            if (s < 0) return;
+            VT()[s].dist = nd;
+            set_birth(s, opv, b);
+            VT()[s].enter = hc.twin;
+            VT()[s].sslot = -1;
+            if (hc.vflags & kVertSaddleGE) ppush(nd, opv, level, b);
+        } while (cur != start && cur != -1);
+        if (init) {
+            uint32_t h;
+            int4 k;
+            double od;
+            int s = vlook(pv, h, k, od);
+            if (s < 0) s = vinsert(pv, h);
+            if (s < 0) return;
+            set_birth(s, pv, 0);
+            VT()[s].dist = 0.0;
+            VT()[s].enter = -1;
+            VT()[s].sslot = -1;
+        }
+    }
+
+    // Process the entry take() popped.  All lanes of `amask` call this
+    // together, each with an entry of the same kind, and meet at each
+    // __syncwarp, so the phases run converged; a lane with nothing to do (an
+    // outdated entry, a boundary edge, a full table) only predicates its work
+    // off.  Both kinds end in the same loop that builds and pushes windows.
+    //
+    // A window crosses the face e0 -> e1 -> e2 beyond it (e0 = twin of its
+    // half-edge) with vertices A = v0(e0), B = v1(e0) and the opposite vertex
+    // C = v1(e1).  The child on e1 (B->C) tests its validity against B, C, A
+    // and the child on e2 (C->A) against C, A, B, so the three distances are
+    // probed once, in parallel with the split entry of e0.
+    __device__ __forceinline__ void act(const int kind, unsigned amask) {
+        const DevMesh& M = C.M;
         pk_valid = false;
-        const bool proc = pk_proc;
-        const WinEntry t = pk_w();
-        WinPay pay;
-        pay.cross = -1;
-        pay.level = 0;
-        if (proc) pay = WP()[t.sb & 0xFFFF];  // issued before the sift-down
-        wpop();
+        const bool window = kind == kActWindow;
+        const double tkey = g_lane_smem.pkey[threadIdx.x];
+        const int tid = g_lane_smem.pid[threadIdx.x];
+        const uint32_t tbits = g_lane_smem.pbits[threadIdx.x];
+        bool live = pk_proc;
+        // what the windows to push have in common
+        double psd = tkey;
+        int level, birth;
+        // window: the face and the split
+        WinPay win;
+        int e1 = 0, e2 = 0;
+        int tw1 = 0, tw2 = 0;
+        double l0 = 0.0, l1 = 0.0, l2 = 0.0, interX = 0.0;
+        double2 v2 = make_double2(0.0, 0.0);
+        double dA = 0.0, dB = 0.0, dC = 0.0;
+        bool keep0 = false, keep1 = false, both = false;
+        // pseudo-source: the fan
+        int startEdge = -1, endEdge = -1;
+        if (window) {
+            copy_async_wait();
+            {
+                const int4 a = g_lane_smem.pay[0][threadIdx.x], b = g_lane_smem.pay[1][threadIdx.x],
+                           c = g_lane_smem.pay[2][threadIdx.x];
+                win.b0 = __hiloint2double(a.y, a.x);
+                win.b1 = __hiloint2double(a.w, a.z);
+                win.sx = __hiloint2double(b.y, b.x);
+                win.sy = __hiloint2double(b.w, b.z);
+                win.psd = __hiloint2double(c.y, c.x);
+                win.cross = c.z;
+                win.level = c.w;
+            }
+            live = live && !(win.level > M.nf);
+            if (live) ++st_windows();
+            psd = win.psd;
+            level = win.level + 1;
+            birth = (int)(signed char)(tbits >> 16);
+            const int e0 = win.cross;
+            const bool on = live && e0 != -1;
+            int Cv = 0;
+            int vfl = 0;
+            uint32_t hA = 0, hB = 0, hC = 0, hS = 0;
+            int4 kA = make_int4(0, 0, 0, 0), kB = kA, kC = kA, kS = kA;
+            double2 sdx = v2;
+            int sC = -1, sS = -1, A = 0, B = 0;
+            if (on) {
+                e1 = nxt(e0);
+                e2 = nxt(e1);
+                const HeRec h0 = ld_he(M.he, e0), h1 = ld_he(M.he, e1), h2 = ld_he(M.he, e2);
+                v2 = ld_apex(M.geo, e0);
+                A = h0.v0;
+                B = h0.v1;
+                Cv = h1.v1;
+                vfl = h1.vflags;
+                l0 = h0.len;
+                l1 = h1.len;
+                l2 = h2.len;
+                tw1 = h1.twin;
+                tw2 = h2.twin;
+                if constexpr (!kCoop) {
+                    vfirst(A, hA, kA, dA);
+                    vfirst(B, hB, kB, dB);
+                    vfirst(Cv, hC, kC, dC);
+                    sfirst(e0, hS, kS, sdx);
+                    vfinish(A, hA, kA, dA);
+                    vfinish(B, hB, kB, dB);
+                    sC = vfinish(Cv, hC, kC, dC);
+                    sS = sfinish(e0, hS, kS, sdx);
+                }
+            }
+            if constexpr (kCoop) {  // the four lookups in one group probe (on is the same in every thread)
+                ProbeR ra, rb, rc, rs;
+                coop_probe4(probe_q(VT(), C.vcap_log2, (uint32_t)A, on), probe_q(VT(), C.vcap_log2, (uint32_t)B, on),
+                            probe_q(VT(), C.vcap_log2, (uint32_t)Cv, on), probe_q(ST(), C.scap_log2, (uint32_t)e0, on),
+                            epoch, ra, rb, rc, rs);
+                dA = ra.slot >= 0 ? __hiloint2double(ra.tail.y, ra.tail.x) : DBL_MAX;
+                dB = rb.slot >= 0 ? __hiloint2double(rb.tail.y, rb.tail.x) : DBL_MAX;
+                dC = rc.slot >= 0 ? __hiloint2double(rc.tail.y, rc.tail.x) : DBL_MAX;
+                sC = rc.slot;
+                kC = rc.head;
+                hC = (uint32_t)(rc.slot >= 0 ? rc.slot : rc.empty);
+                sS = rs.slot;
+                hS = (uint32_t)(rs.slot >= 0 ? rs.slot : rs.empty);
+                sdx = rs.slot >= 0 ? make_double2(__hiloint2double(rs.tail.y, rs.tail.x),
+                                                  __hiloint2double(rs.tail.w, rs.tail.z))
+                                   : make_double2(DBL_MAX, DBL_MAX);
+            }
+            __syncwarp(amask);
+            keep0 = keep1 = on;
+            if (on) {
+                interX = v2.x - v2.y * (v2.x - win.sx) / (v2.y - win.sy);
+                if (interX <= win.b0) {
+                    keep0 = false;  // right child only
+                } else if (interX >= win.b1) {
+                    keep1 = false;  // left child only
+                } else {
+                    both = true;
+                    const double D = hyp(v2.x - win.sx, v2.y - win.sy) + win.psd;
+                    const double sd = sdx.x;
+                    if (D > sd && exceeds_rel(D, sd)) {  // one angle, one split
+                        keep0 = sdx.y < interX;
+                        keep1 = !keep0;
+                    } else {
+                        int ssl = sS;
+                        bool ok = true;
+                        if (D < sd) {
+                            if (ssl < 0) ssl = sinsert(e0, hS);  // the lookup's chain ended at the empty slot
+                            if (ssl < 0) {
+                                ok = false;  // table full: the source goes to the retry pass
+                            } else {
+                                ST()[ssl].dist = D;
+                                ST()[ssl].psrc = tid;
+                                ST()[ssl].x = l0 - interX;
+                            }
+                        }
+                        if (ok && D < dC) {
+                            if (dC == DBL_MAX) ++total;
+                            const int s = sC >= 0 ? sC : vinsert(Cv, hC);
+                            if (s < 0) {
+                                ok = false;
+                            } else {
+                                const int b = (int)(signed char)((sC >= 0 ? kC.w : -1) + 1);
+                                set_birth(s, Cv, b);
+                                VT()[s].dist = D;
+                                VT()[s].enter = e0;
+                                VT()[s].sslot = ssl;  // D < dC <= split distance: the entry was just written
+                                dC = D;  // the children's tests read the updated distance
+                                if (vfl & kVertSaddleGT) ppush(D, Cv, level, b);
+                            }
+                        }
+                        if (!ok) keep0 = keep1 = false;
+                    }
+                }
+            }
+        } else {
+            const int plevel = (int)(tbits >> 8);
+            birth = (int)(signed char)(tbits & 0xFF);
+            level = pk_init ? 0 : plevel + 1;
+            if (!pk_init) {
+                live = live && !(plevel >= M.nf);
+                if (live) {
+                    ++st_pseudos();
+                    live = fan_range(tid, startEdge, endEdge);
+                }
+            } else {
+                startEdge = endEdge = __ldg(&M.vr[tid].first);
+                if (startEdge < 0) {  // isolated vertex: the reference indexes edges[-1]
+                    flags |= kFlagUndefined;
+                    live = false;
+                }
+            }
+            keep0 = live;  // more of the fan to come
+        }
         __syncwarp(amask);
-        const bool live = proc && !(pay.level > C.M.nf);
-        if (live) ++st_windows();
-        propagate(pay, t.psrc, (int)(signed char)(t.sb >> 16), live, amask);
+
+        // Build, test and push the windows: the two children of a window (the
+        // tests read only the three distances, which a push does not change),
+        // or the fan of a pseudo-source from startEdge round to endEdge.
+        int c = 0;
+#pragma unroll 1
+        for (;; ++c) {
+            bool keep;
+            if (window) {
+                if (c == 2) break;
+                keep = c == 0 ? keep0 : keep1;
+            } else {
+                if (keep0 && startEdge < 0) {  // the reference reads edges[-1] here
+                    flags |= kFlagUndefined;
+                    keep0 = false;
+                }
+                keep = keep0;
+            }
+            if (!__any_sync(amask, keep)) {
+                if (window) continue;
+                break;
+            }
+            NewWin W;
+            if (keep) {
+                double b0, b1, d0, d1;
+                double2 top = make_double2(0.0, 0.0);
+                if (window) {
+                    // ICHDevice::BuildWindow (ICHDevice.cu:957-973).  Child 0:
+                    // frame (0,0) -> apex; child 1: apex -> (l0,0)
+                    const bool left = c == 0;
+                    top = ld_top(M.geo, left ? e1 : e2);
+                    const double f0x = left ? 0.0 : v2.x, f0y = left ? 0.0 : v2.y;
+                    const double f1x = left ? v2.x : l0, f1y = left ? v2.y : 0.0;
+                    const bool fix0 = !left && both, fix1 = left && both;
+                    const double t0 = fix0 ? 1.0 : isect(win.sx, win.sy, win.b0, 0.0, f0x, f0y, f1x, f1y);
+                    const double t1 = fix1 ? 0.0 : isect(win.sx, win.sy, win.b1, 0.0, f0x, f0y, f1x, f1y);
+                    const double elen = left ? l1 : l2;
+                    b0 = (1 - t0) * elen;
+                    b1 = (1 - t1) * elen;
+                    double px = f0x * t0 + f1x * (1 - t0), py = f0y * t0 + f1y * (1 - t0);
+                    d0 = hyp(win.sx - px, win.sy - py);
+                    px = f0x * t1 + f1x * (1 - t1);
+                    py = f0y * t1 + f1y * (1 - t1);
+                    d1 = hyp(win.sx - px, win.sy - py);
+                    W.p.cross = left ? tw1 : tw2;
+                } else {
+                    const int we = nxt(startEdge);
+                    const HeRec hs = ld_he(M.he, startEdge), hw = ld_he(M.he, we), hn = ld_he(M.he, nxt(we));
+                    b0 = 0.0;
+                    b1 = hw.len;
+                    d0 = hs.len;
+                    d1 = hn.len;
+                    W.p.cross = hw.twin;
+                    // Initialize turns the other way round the vertex and ends at a boundary
+                    startEdge = pk_init ? (hs.twin < 0 ? -1 : nxt(hs.twin)) : hn.twin;
+                    if (startEdge == endEdge || (pk_init && startEdge < 0)) keep0 = false;
+                    if (c > 1 << 20) { flags |= kFlagWatchdog; keep0 = live = false; }
+                }
+                finish_window(b0, b1, d0, d1, psd, W);
+                W.p.level = level;
+                if (window)
+                    keep = c == 0 ? valid_window(W, true, dB, dC, dA, l1, top.x, top.y)
+                                  : valid_window(W, false, dC, dA, dB, l2, top.x, top.y);
+            }
+            __syncwarp(amask);
+            if (keep) wpush(W, tid, birth);
+            __syncwarp(amask);
+        }
+        if (!window) {
+            if (live) ring(tkey, tid, level - (pk_init ? 0 : 1), pk_init);
+            __syncwarp(amask);
+        }
         if (live && C.K != -1 && total >= C.K) done = true;
     }
 
-    __device__ void act_pseudo(unsigned amask) {
-        pk_valid = false;
-        const bool proc = pk_proc;
-        const PsEntry t = pk_p();
-        ppop();
-        __syncwarp(amask);
-        const int level = (int)(t.lb >> 8);
-        const bool live = proc && !(level >= C.M.nf);
-        if (live) ++st_pseudos();
-        gen_sub_wins(t.key, t.vert, level, (int)(signed char)(t.lb & 0xFF), live, amask);
-        if (live && C.K != -1 && total >= C.K) done = true;
-    }
-
-    // peek + act for one lane on its own (or, cooperative, for the whole
-    // warp on its source); true when finished.
+    // take + act for one lane on its own (or, cooperative, for the whole
+    // warp on its source); true when finished.  A lane stepping on its own
+    // gains nothing from dropping outdated entries inside take().
     __device__ bool step() {
         const unsigned self = kCoop ? 0xFFFFFFFFu : 1u << (threadIdx.x & 31);
-        const int a = peek<0>();
+        const int a = take<0>();
         if (a == kActDone) return true;
-        if (a == kActWindow) act_window(self);
-        else act_pseudo(self);
+        act(a, self);
         return false;
     }
 };

@@ -18,7 +18,7 @@ struct alignas(32) HeRec {
     int32_t v0;      // edges[e].verts[0]
     int32_t v1;      // edges[e].verts[1]
     int32_t twin;    // -1 on the boundary
-    int32_t pad;
+    int32_t vflags;  // saddle flags of v1
     double len;      // edges[e].edgeLen
     double corner;   // corner angle of face(e) at v0(e): acos of the law of cosines, clamped
 };
