@@ -89,6 +89,9 @@ struct PhaseOut {
     // 1: once the work queue is drained, a warp left with one running lane
     // finishes that lane's source in the cooperative form
     int32_t coop_tail;
+    // lanes of each warp that run sources (the lane scratch is laid out for
+    // them alone: lane l of warp w has the scratch of index w * warp_lanes + l)
+    int32_t warp_lanes;
 };
 
 template <class LaneType>
@@ -123,7 +126,7 @@ __device__ void finish_warp(LaneType& L, const PhaseOut& O, int v, unsigned amas
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     const DevMesh& M = L.C.M;
-    const int warp_base = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+    const int warp_base = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * O.warp_lanes;
     unsigned todo = amask;
     while (todo) {
         const int o = __ffs(todo) - 1;
@@ -232,13 +235,12 @@ __device__ void finish_warp(LaneType& L, const PhaseOut& O, int v, unsigned amas
 // lane while 31 idle.
 __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
     constexpr unsigned kFull = 0xFFFFFFFFu;
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int wbase = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * O.warp_lanes;
     if (threadIdx.x < 32 && (int)blockIdx.x < O.coop_warps) {
         // Cooperative phase: the whole warp on one heavy source at a time,
         // its heaps in shared memory, its pool and tables in the scratch of
         // the warp's first lane.
         extern __shared__ __align__(16) unsigned char s_heaps[];
-        const int wbase = gtid & ~31;
         CoopLane W(C, wbase);
         W.sheap = reinterpret_cast<HeapEntry*>(s_heaps);
         for (;;) {
@@ -255,8 +257,10 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
         if ((threadIdx.x & 31) == 0) W.save_epoch(wbase);
         __syncwarp();
     }
-    Lane L(C, gtid);
-    int r = O.coop_n + atomicAdd(O.work, 1);
+    const bool runs = (int)(threadIdx.x & 31) < O.warp_lanes;
+    const int lid = wbase + (runs ? (int)(threadIdx.x & 31) : 0);
+    Lane L(C, lid);
+    int r = runs ? O.coop_n + atomicAdd(O.work, 1) : O.nsrc;
     int v = r < O.nsrc ? O.order[r] : -1;
     if (v >= 0) L.begin(v, false);
     int waited = 0;
@@ -275,9 +279,11 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
             const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
             chosen = (c0 >= c1 && c0 >= c2) ? Lane::kActWindow : (c1 >= c2 ? Lane::kActPseudo : Lane::kActDone);
         }
-        if (O.coop_tail && m2 == 0 && __popc(m0 | m1) == 1 && __ballot_sync(kFull, v < 0) == ~(m0 | m1)) {
-            // The queue is drained (every other lane found it empty) and one
-            // lane still runs a source: the whole warp adopts it below.
+        if (O.coop_tail && O.warp_lanes > 1 && m2 == 0 && __popc(m0 | m1) == 1 &&
+            __ballot_sync(kFull, v < 0) == ~(m0 | m1)) {
+            // The queue is drained (every other lane that runs sources found it
+            // empty) and one lane still runs a source: the whole warp adopts it
+            // below.
             adopt = __ffs(m0 | m1) - 1;
             break;
         }
@@ -296,9 +302,9 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
             ++waited;
         }
     }
-    L.save_epoch(gtid);  // adoption below keeps lane `adopt`'s epoch: no begin() runs there
+    if (runs) L.save_epoch(lid);  // adoption below keeps lane `adopt`'s epoch: no begin() runs there
     if (adopt >= 0) {
-        CoopLane W(C, blockIdx.x * blockDim.x + (threadIdx.x & ~31));
+        CoopLane W(C, wbase);
         W.adopt(L, adopt);
         while (!W.step()) {
         }
@@ -1012,7 +1018,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         SVG_CUDA(cudaGetDevice(&dev0));
         SVG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev0));
         SVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ich_batched, 128, 0));
-        probe_lanes = std::max(1, per_sm) * sms * 128;
+        probe_lanes = std::max(1, std::min(per_sm, 2)) * sms * 128;  // measured with two blocks per SM
     }
     if (!plain && o.heavy_first == 2 && nsrc > 0 && K >= 160 &&
         (int64_t)nsrc <= (int64_t)kProbeSourcesPerLane * probe_lanes &&
@@ -1097,12 +1103,25 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         if (per_sm > 2 && 4 * (int64_t)nsrc < (int64_t)7 * per_sm * prop.multiProcessorCount * tpb) per_sm = 2;
         blocks = std::max(1, per_sm) * prop.multiProcessorCount;
     }
-    int64_t want_blocks = (nsrc + tpb - 1) / tpb;
-    if (!plain) blocks = (int)std::min<int64_t>(blocks, std::max<int64_t>(1, want_blocks));
-    lay.lanes = blocks * tpb;
-    while (lay.lanes > 32 && (int64_t)(lane_bytes(lay) * lay.lanes) > budget) {
+    // Fewer sources than lanes: every warp gets as few of them as spreads them
+    // over all warps.  A warp's step waits for its slowest lane and runs every
+    // branch some lane takes: on the idle GPU a step took 4.1 us with one
+    // active lane, 8.0 with 4, 9.7 with 8 and 13.2 with 32.  Measured against
+    // full warps: 609 sources at K = 20 1.06 -> 0.34 ms, 5K at K = 50
+    // 4.33 -> 2.84 ms, 12K at K = 200 69.2 -> 50.1 ms, 30K at K = 100
+    // 16.6 -> 15.6 ms.
+    int warp_lanes = 32;
+    if (!plain) {
+        const int64_t warps = (int64_t)blocks * (tpb / 32);
+        warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps - 1) / warps));
+        const int64_t per_block = (int64_t)(tpb / 32) * warp_lanes;
+        blocks = (int)std::min<int64_t>(blocks, std::max<int64_t>(1, (nsrc + per_block - 1) / per_block));
+    }
+    const int block_lanes = plain ? tpb : (tpb / 32) * warp_lanes;
+    lay.lanes = blocks * block_lanes;
+    while (blocks > 1 && (int64_t)(lane_bytes(lay) * lay.lanes) > budget) {
         blocks = std::max(1, blocks / 2);
-        lay.lanes = blocks * tpb;
+        lay.lanes = blocks * block_lanes;
     }
     if ((int64_t)(lane_bytes(lay) * lay.lanes) > budget)
         throw SvgError{SVG_ERR_NOMEM, "HBM budget too small for one block of build lanes"};
@@ -1158,12 +1177,12 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                 while (n < head && (double)m->cost[(size_t)ord[(size_t)n]] >= share) ++n;
                 n = std::min<int64_t>(n, lay.lanes / 64);
             }
-            const int64_t warps = (int64_t)lay.lanes / 32;
+            const int64_t warps = (int64_t)blocks * (tpb / 32);
             coop_n = (int32_t)n;
             // one cooperative warp per block at most (warp 0, whose block holds its heaps)
             coop_warps = (int32_t)std::min<int64_t>(
                 {o.coop_warps > 0 ? (int64_t)o.coop_warps : std::max<int64_t>(1, n / 2), n, warps / 2,
-                 (int64_t)lay.lanes / tpb});
+                 (int64_t)blocks});
             if (coop_warps <= 0) coop_n = 0;
         }
         SVG_CUDA(cudaMemcpyAsync(d_order, ord.data(), sizeof(int32_t) * (size_t)nsrc, cudaMemcpyHostToDevice, st));
@@ -1212,6 +1231,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     O.coop_warps = coop_warps;
     O.coop_work = d_work + 4;
     O.coop_tail = o.coop_tail != 0 ? 1 : 0;
+    O.warp_lanes = warp_lanes;
 
     cudaEvent_t ev[4];
     for (auto& e : ev) SVG_CUDA(cudaEventCreate(&e));
@@ -1285,17 +1305,21 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                 C2.scap_log2 = l2.scap_log2;
                 C2.vlimit = l2.vlimit;
                 C2.slimit = (int32_t)(((int64_t)3 << l2.scap_log2) / 4);
-                int tb2 = 64;
-                int bl2 = (int)std::min<int64_t>((retry_n + tb2 - 1) / tb2, (int64_t)prop.multiProcessorCount * 4);
-                l2.lanes = bl2 * tb2;
-                while (l2.lanes > 32 && (int64_t)(lane_bytes(l2) * l2.lanes) > budget) {
+                // spread over the warps as in the first pass
+                const int tb2 = 64;
+                int bl2 = prop.multiProcessorCount * 4;
+                const int wl2 = (int)std::min<int64_t>(32, ((int64_t)retry_n + 2 * bl2 - 1) / (2 * bl2));
+                bl2 = (int)std::min<int64_t>(bl2, ((int64_t)retry_n + 2 * wl2 - 1) / (2 * wl2));
+                l2.lanes = bl2 * 2 * wl2;
+                while (bl2 > 1 && (int64_t)(lane_bytes(l2) * l2.lanes) > budget) {
                     bl2 = std::max(1, bl2 / 2);
-                    l2.lanes = bl2 * tb2;
+                    l2.lanes = bl2 * 2 * wl2;
                 }
                 carve(g_arena[1], l2, C2, st);
                 scratch_bytes += (int64_t)(lane_bytes(l2) * l2.lanes);
                 PhaseOut O2 = O;
                 O2.coop_n = 0;
+                O2.warp_lanes = wl2;
                 O2.coop_warps = 0;
                 O2.order = d_retry;
                 O2.nsrc = retry_n;

@@ -51,6 +51,21 @@ def test_build_matches_reference_golden(name, K, mode):
     assert st["watchdog_sources"] == 0
 
 
+@pytest.mark.parametrize("n,blocks", [(1, 0), (2, 0), (4, 1), (5, 1), (9, 1), (127, 1), (128, 1), (129, 1), (300, 2),
+                                      (1185, 0), (1500, 0)])
+def test_sources_spread_over_warps_keep_their_rows(n, blocks):
+    """Fewer sources than lanes run a few to a warp (1, 2, 3, ... 32 active
+    lanes, one source more than the lanes, whole warps with none): the rows of
+    the plain form, whose sources run one per thread."""
+    pos, faces = meshgen.config_mesh(0, 0.25)
+    out = []
+    for mode, kw in ((MODE_PLAIN, {}), (MODE_BATCHED, dict(blocks=blocks))):
+        off, nodes, st, _, _ = gpu_build(pos, faces, 40, mode, source_begin=100, source_end=100 + n, **kw)
+        assert st["sources"] == n
+        out.append((off, nodes))
+    assert compare_rows(*out[0], *out[1]) == []
+
+
 def coop_build(pos, faces, K, coop_warps=8, coop_sources=None, **kw):
     """Batched build whose work order comes from a first build's per-source
     costs, with the heaviest `coop_sources` (default: every source) run by
