@@ -95,10 +95,10 @@ typedef struct svg_build_opts {
     int32_t threads_per_block;/* 0 = autotuned (batched) / 128 (plain, SVG.cuh:11) */
     int32_t blocks;           /* 0 = autotuned (batched) / 64 (plain, SVG.cuh:10) */
     int32_t with_paths;       /* 1 = also produce the path-end fields of svg_node */
-    int32_t heavy_first;      /* batched: order the work queue heaviest first, by the per-source cost of the
-                                 mesh's previous build at this K (1), or, lacking one, of a probe build at
-                                 K/10 when K >= 160 and a launch's lanes get at most 4 sources each
-                                 (2, the default); 0: vertex order */
+    int32_t heavy_first;      /* batched, more sources than a launch's lanes: order the work queue heaviest
+                                 first, by the per-source cost of the mesh's previous build at this K (1), or,
+                                 lacking one, of a probe build at K/10 when K >= 160 and the lanes get at most
+                                 8/3 sources each (2, the default); 0: vertex order */
     int64_t hbm_budget;       /* bytes of scratch the build may hold (0 = automatic) */
     int32_t source_begin;     /* build rows for sources [source_begin, source_end) only; */
     int32_t source_end;       /* 0,0 = all vertices */

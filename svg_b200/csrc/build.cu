@@ -77,7 +77,7 @@ struct PhaseOut {
     int32_t* st_windows;
     int32_t* st_maxq;
     int32_t* st_flags;
-    unsigned long long* acc;       // windows, generated, pseudo-sources, queue-drop sources
+    unsigned long long* acc;       // windows, generated, pseudo-sources, largest queues, largest source's windows
     // Cooperative warps: warp 0 of each of the first coop_warps blocks takes
     // the heaviest sources order[0 .. coop_n) one at a time from its own
     // queue head (coop_work) and runs each with the whole warp, its two heaps
@@ -109,6 +109,7 @@ __device__ void record_stats(const LaneType& L, const PhaseOut& O, int v) {
     atomicAdd(&O.acc[2], (unsigned long long)L.st_pseudos());
     atomicMax(reinterpret_cast<unsigned long long*>(&O.acc[3]), (unsigned long long)L.st_maxw());
     atomicMax(reinterpret_cast<unsigned long long*>(&O.acc[4]), (unsigned long long)L.st_maxp());
+    atomicMax(reinterpret_cast<unsigned long long*>(&O.acc[5]), (unsigned long long)L.st_windows());
 }
 
 // End of the sources of the lanes in `amask` (they finished in this step):
@@ -583,9 +584,24 @@ __global__ void k_compact(const int32_t* order, int32_t nsrc, int32_t K, const i
     }
 }
 
-__global__ void k_iota(int32_t* o, int32_t n, int32_t base) {
+// Where entry i of a launch's first wave stands in the list it is taken from:
+// the lanes of a warp fetch consecutive entries, and lane l of warp w gets
+// entry l * warps + w, so that a warp holds sources from all over the list.
+// In cost order, each warp then has a few heavy sources whose lanes run on
+// with fewer and fewer neighbours (a warp of one active lane steps three times
+// as fast as a full one), instead of 32 heavy ones that slow each other to
+// the end; in vertex order, neighbours of similar cost are spread likewise.
+// Kernel time, consecutive -> strided: 30K height field K = 500 317 -> 233 ms,
+// 12K K = 200 48.6 -> 39.6 ms, 73K K = 500 531 -> 438 ms; 30K torus K = 100
+// 14.5 -> 13.5 ms; launches of many waves are not affected.
+__host__ __device__ inline int64_t strided(int64_t i, int64_t warps, int64_t warp_lanes) {
+    return i < warps * warp_lanes ? (i % warp_lanes) * warps + i / warp_lanes : i;
+}
+
+// Sources in vertex order, the first wave strided (warps 0: not).
+__global__ void k_order(int32_t* o, int32_t n, int32_t base, int32_t warps, int32_t warp_lanes) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) o[i] = base + i;
+    if (i < n) o[i] = base + (int32_t)strided(i, warps, warp_lanes);
 }
 
 // ------------------------------------------------------------------ host
@@ -746,7 +762,7 @@ svg_build_opts effective_options(const svg_mesh* m, const svg_build_opts& o) {
 namespace {
 // Flag tallies of a finished build; per-source costs kept on the mesh for
 // the next build's order.
-void record_counts(svg_mesh* m, svg_graph* g, int32_t K, int32_t sb, int32_t se, bool plain) {
+void record_counts(svg_mesh* m, svg_graph* g, int32_t K, int32_t sb, int32_t se, bool plain, int64_t max_windows) {
     const int32_t nv = g->nv;
     svg_build_stats& S = g->stats;
     std::vector<int32_t> fl((size_t)nv);
@@ -761,6 +777,7 @@ void record_counts(svg_mesh* m, svg_graph* g, int32_t K, int32_t sb, int32_t se,
         }
         for (int32_t v = sb; v < se; ++v) m->cost[(size_t)v] = w[(size_t)v];
         if (sb == 0 && se == nv) m->cost_probe = false;
+        m->cost_even = 2 * max_windows * S.sources <= 3 * S.windows;  // largest at most 1.5 times the mean
     }
     for (int32_t f : fl) {
         if (f & 1) ++S.queue_drop_sources;
@@ -840,7 +857,7 @@ bool replay_graph(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
     S.coop_sources = bg->coop_n;
     S.coop_warps = bg->coop_warps;
     S.graph_replayed = 1;
-    record_counts(m, g, o.K, bg->sb, bg->se, false);
+    record_counts(m, g, o.K, bg->sb, bg->se, false, (int64_t)acc[5]);
     return true;
 }
 
@@ -1007,21 +1024,22 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     // K/10 (a few per cent of the work) supplies the per-source estimate.  It
     // runs before this build takes the scratch arena, which the probe reuses.
     // The order only pays where a lane gets few sources, so that the last,
-    // heaviest ones set the build's length: up to kProbeSourcesPerLane per
-    // lane of a full launch (measured: 6 % faster on a 72.9K-vertex height
-    // field at K = 500 with 1.9 sources per lane, 4 % slower on a 750K-vertex
-    // torus with 20).
-    constexpr int kProbeSourcesPerLane = 4;
-    int probe_lanes = 0;
+    // heaviest ones set the build's length: up to 8/3 per lane of a full launch
+    // (151K sources; measured: 6 % faster on a 72.9K-vertex height field at
+    // K = 500, 4 % slower on a 750K-vertex torus).  And a launch with a lane
+    // for every source needs no costs: the strided vertex order is as fast as
+    // the cost order there (30K height field K = 500 235 / 233 ms, 45K K = 200
+    // 62.8 / 64.8 ms).
+    int full_lanes = 0;
     if (!plain && o.heavy_first == 2) {
         int per_sm = 0, dev0 = 0, sms = 0;
         SVG_CUDA(cudaGetDevice(&dev0));
         SVG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev0));
         SVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ich_batched, 128, 0));
-        probe_lanes = std::max(1, std::min(per_sm, 2)) * sms * 128;  // measured with two blocks per SM
+        full_lanes = std::max(1, per_sm) * sms * 128;
     }
-    if (!plain && o.heavy_first == 2 && nsrc > 0 && K >= 160 &&
-        (int64_t)nsrc <= (int64_t)kProbeSourcesPerLane * probe_lanes &&
+    if (!plain && o.heavy_first == 2 && nsrc > full_lanes && K >= 160 &&
+        3 * (int64_t)nsrc <= 8 * (int64_t)full_lanes &&
         !(m->cost_K == K && (int32_t)m->cost.size() == nv)) {
         svg_build_opts po = o;
         po.K = K / 10;
@@ -1094,17 +1112,16 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     } else if (blocks <= 0) {
         int per_sm = 0;
         SVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ich_batched, tpb, 0));
-        // A third block per SM raises the throughput but also the time of each
-        // lane's step, and with few sources per lane the heaviest sources' steps
-        // are the build's length.  Measured, two blocks against three: 73K
-        // sources (1.3 per lane of three blocks) 31.0 / 32.2 ms at K = 100 and
-        // 455 / 530 ms at K = 500; 120K sources (2.1) 51.1 / 42.0 ms at K = 100
-        // and 162 / 140 ms at K = 200; 750K sources 277 / 240 ms at K = 100.
-        if (per_sm > 2 && 4 * (int64_t)nsrc < (int64_t)7 * per_sm * prop.multiProcessorCount * tpb) per_sm = 2;
+        // With at most 8 sources to a warp of two blocks per SM, a third block
+        // only adds warps that wait on the same memory: 5K sources at K = 50
+        // 2.74 ms with two, 2.83 with three; 12K at K = 200 39.5 / 40.0 ms.
+        // From there three are as fast or faster: 30K torus K = 100 13.9 / 13.5
+        // ms, 73K height field K = 500 441 / 411 ms, 750K torus 271 / 229 ms.
+        if (per_sm > 2 && nsrc <= 8 * 2 * prop.multiProcessorCount * (tpb / 32)) per_sm = 2;
         blocks = std::max(1, per_sm) * prop.multiProcessorCount;
     }
-    // Fewer sources than lanes: every warp gets as few of them as spreads them
-    // over all warps.  A warp's step waits for its slowest lane and runs every
+    // Active lanes per warp.  Fewer sources than lanes: every warp gets as few
+    // of them as spreads them over all warps.  A warp's step waits for its slowest lane and runs every
     // branch some lane takes: on the idle GPU a step took 4.1 us with one
     // active lane, 8.0 with 4, 9.7 with 8 and 13.2 with 32.  Measured against
     // full warps: 609 sources at K = 20 1.06 -> 0.34 ms, 5K at K = 50
@@ -1112,8 +1129,19 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     // 16.6 -> 15.6 ms.
     int warp_lanes = 32;
     if (!plain) {
+        // More sources than lanes: where a nearly empty last wave would follow
+        // full ones, the waves are made equal by using fewer lanes of each warp.
+        // That pays where all sources cost about the same (a lane starts its
+        // last source when the others do) and, through the smaller scratch in
+        // flight, at large K.  Full / equal waves: 73K torus K = 100 29.0 /
+        // 28.0 ms, K = 500 288 / 268 ms, 120K K = 200 125 / 117 ms; 73K height
+        // field K = 500 438 / 411 ms, but K = 100 26.2 / 28.7 ms and 120K
+        // K = 200 134 / 141 ms.
         const int64_t warps = (int64_t)blocks * (tpb / 32);
-        warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps - 1) / warps));
+        const bool costs = m->cost_K == K && (int32_t)m->cost.size() == nv;
+        const bool equal = K >= 300 || (costs && m->cost_even);
+        const int64_t waves = equal ? std::max<int64_t>(1, (nsrc + 32 * warps - 1) / (32 * warps)) : 1;
+        warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps * waves - 1) / (warps * waves)));
         const int64_t per_block = (int64_t)(tpb / 32) * warp_lanes;
         blocks = (int)std::min<int64_t>(blocks, std::max<int64_t>(1, (nsrc + per_block - 1) / per_block));
     }
@@ -1138,7 +1166,10 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     b_order.reserve(sizeof(int32_t) * (size_t)std::max(nsrc, 1));
     int32_t* d_order = b_order.as<int32_t>();
     bool ordered = false;
-    if (!plain && o.heavy_first && m->cost_K == K && (int32_t)m->cost.size() == nv && nsrc > 0) {
+    const bool one_wave = nsrc <= lay.lanes;
+    const int32_t wave_warps = plain ? 0 : std::min(nsrc, lay.lanes) / warp_lanes;
+    if (!plain && o.heavy_first && m->cost_K == K && (int32_t)m->cost.size() == nv && nsrc > 0 &&
+        (!one_wave || o.coop_sources != 0)) {
         // The heaviest sources, two per lane, go first (they would otherwise
         // set the tail); the rest keep vertex order, so that the sources in
         // flight together stay neighbours on the mesh and share its lines in L2
@@ -1151,9 +1182,11 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         std::stable_sort(byc.begin(), byc.end(),
                          [&](int32_t a, int32_t b) { return m->cost[(size_t)a] > m->cost[(size_t)b]; });
         std::vector<char> taken((size_t)nsrc, 0);
+        // the cooperative warps take their sources from the front, in cost order
+        const int32_t stride_warps = o.coop_sources != 0 ? 0 : wave_warps;
         for (int64_t i = 0; i < head; ++i) {
-            ord[(size_t)i] = byc[(size_t)i];
-            taken[(size_t)(byc[(size_t)i] - sb)] = 1;
+            ord[(size_t)i] = byc[(size_t)strided(i, stride_warps, warp_lanes)];
+            taken[(size_t)ord[(size_t)i] - (size_t)sb] = 1;
         }
         int64_t k = head;
         for (int32_t i = 0; i < nsrc; ++i)
@@ -1189,7 +1222,8 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         SVG_CUDA(cudaStreamSynchronize(st));
         ordered = true;
     }
-    if (nsrc > 0 && !ordered) k_iota<<<(nsrc + 255) / 256, 256, 0, st>>>(d_order, nsrc, sb);
+    if (nsrc > 0 && !ordered)
+        k_order<<<(nsrc + 255) / 256, 256, 0, st>>>(d_order, nsrc, sb, wave_warps, warp_lanes);
     // misc: work, retry_n, acc[8], cand_used ; retry list ; cand_n ; deg
     // retry list: room for the first pass's failures and, after them, the retry pass's
     size_t retry_bytes = align_up(sizeof(int32_t) * 2 * (size_t)std::max(nsrc, 1));
@@ -1235,7 +1269,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
 
     cudaEvent_t ev[4];
     for (auto& e : ev) SVG_CUDA(cudaEventCreate(&e));
-    int launches = 1;  // iota
+    int launches = 1;  // the work order
     SVG_CUDA(cudaEventRecord(ev[0], st));
 
     DevBuf b_padj, b_pdist, b_ppath, b_tails;
@@ -1432,7 +1466,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     S.coop_sources = coop_n;
     S.coop_warps = coop_warps;
     (void)t03;
-    record_counts(m, g, K, sb, se, plain);
+    record_counts(m, g, K, sb, se, plain, (int64_t)acc[5]);
     if (o.graph && !plain && nsrc > 0 && retry_n == 0 && cap_attempts == 0) {
         CapturePlan P;
         P.C = C;

@@ -81,6 +81,8 @@ struct svg_mesh {
     std::vector<int32_t> cost;
     // the costs are a K/10 probe build's stand-in, not a build at cost_K
     bool cost_probe = false;
+    // the costliest source of that build took at most 1.5 times the mean
+    bool cost_even = false;
     // the last build captured as a CUDA graph (opts.graph), replayed by later
     // builds with the same options
     std::shared_ptr<svgb::BuildGraph> build_graph;

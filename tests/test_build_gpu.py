@@ -66,6 +66,24 @@ def test_sources_spread_over_warps_keep_their_rows(n, blocks):
     assert compare_rows(*out[0], *out[1]) == []
 
 
+@pytest.mark.parametrize("n,blocks", [(128, 1), (129, 1), (255, 1), (257, 1), (700, 2), (1600, 3)])
+def test_strided_work_order_keeps_the_rows(n, blocks):
+    """More sources than a launch's lanes (128 per block), or just as many: the
+    first wave strided over the warps in vertex order, then in the order of the
+    first build's costs; every source is built once, with the plain form's rows."""
+    pos, faces = meshgen.config_mesh(1, 0.2)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(30)
+    s.ConstructSVG(mode=MODE_PLAIN, source_begin=7, source_end=7 + n)
+    want = s.CopySVGToHost()
+    for _ in range(3):
+        st = s.ConstructSVG(blocks=blocks, heavy_first=1, source_begin=7, source_end=7 + n)
+        assert st["sources"] == n
+        assert compare_rows(*s.CopySVGToHost(), *want) == []
+
+
 def coop_build(pos, faces, K, coop_warps=8, coop_sources=None, **kw):
     """Batched build whose work order comes from a first build's per-source
     costs, with the heaviest `coop_sources` (default: every source) run by
