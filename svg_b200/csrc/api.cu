@@ -1,4 +1,5 @@
 // C ABI of svg_b200 (include/svg_b200.h): object lifetime, errors, I/O.
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -147,6 +148,14 @@ DevMesh MeshDev::view() const {
     return v;
 }
 
+// The saddle flags of each half-edge's end vertex, into its record: a window
+// step or a fan then reads them with the half-edge instead of in a further
+// round trip.
+__global__ void k_end_flags(HeRec* he, const VertRec* vr, int32_t ne) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x)
+        he[e].vflags = vr[he[e].v1].flags;
+}
+
 void upload_mesh(svg_mesh* m) {
     if (m->d.uploaded) return;
     const HostMesh& H = m->h;
@@ -168,6 +177,8 @@ void upload_mesh(svg_mesh* m) {
     SVG_CUDA(cudaMemcpyAsync(D.geo, H.geo.data(), sizeof(HeGeo) * (size_t)H.ne, cudaMemcpyHostToDevice, st));
     SVG_CUDA(cudaMemcpyAsync(D.vr, H.vr.data(), sizeof(VertRec) * (size_t)H.nv, cudaMemcpyHostToDevice, st));
     SVG_CUDA(cudaMemcpyAsync(D.pos, H.pos.data(), sizeof(double) * 3 * (size_t)H.nv, cudaMemcpyHostToDevice, st));
+    k_end_flags<<<(int)std::min<int64_t>(((int64_t)H.ne + 255) / 256, 2048), 256, 0, st>>>(D.he, D.vr, H.ne);
+    SVG_CUDA(cudaGetLastError());
     SVG_CUDA(cudaStreamSynchronize(st));
     D.nv = H.nv;
     D.nf = H.nf;

@@ -604,6 +604,102 @@ __global__ void k_order(int32_t* o, int32_t n, int32_t base, int32_t warps, int3
     if (i < n) o[i] = base + (int32_t)strided(i, warps, warp_lanes);
 }
 
+// The work order by cost, on the device: a counting sort of the sources by
+// cost bin (descending), of which the first `head` or so (whole bins) go to
+// the front of the order, the first wave of them strided; the rest follows in
+// vertex order, block by block, so that the sources in flight together stay
+// neighbours on the mesh and share its lines in L2.  Three small launches in
+// place of copying the costs to the host, sorting there and copying the order
+// back (750K sources: 45 ms of a 340 ms build).
+constexpr int kCostBins = 2048;
+struct CostPlan {
+    int32_t start[kCostBins];  // sources in heavier bins: where a bin's run begins
+    int32_t fill[kCostBins];   // histogram, then entries of the bin placed so far
+    int32_t heavy;             // sources in front; bins whose run begins below `head`
+    int32_t rest;              // of the others, placed so far
+};
+struct CostOrder {
+    const int32_t* cost;  // per vertex
+    int32_t sb, nsrc, head, shift;
+    int32_t warps, warp_lanes;
+    CostPlan* plan;
+    int32_t* order;
+    __device__ int bin(int i) const { return min(kCostBins - 1, max(0, cost[sb + i]) >> shift); }
+};
+__global__ void __launch_bounds__(256) k_cost_hist(CostOrder P) {
+    __shared__ int32_t h[kCostBins];
+    for (int b = threadIdx.x; b < kCostBins; b += blockDim.x) h[b] = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nsrc; i += gridDim.x * blockDim.x)
+        atomicAdd(&h[P.bin(i)], 1);
+    __syncthreads();
+    for (int b = threadIdx.x; b < kCostBins; b += blockDim.x)
+        if (h[b]) atomicAdd(&P.plan->fill[b], h[b]);
+}
+__global__ void __launch_bounds__(1024) k_cost_plan(CostOrder P) {  // one block
+    __shared__ int32_t s[1024];
+    const int t = threadIdx.x, hi = kCostBins - 1 - 2 * t, lo = hi - 1;  // this thread's bins, heavier first
+    const int32_t nh = P.plan->fill[hi], nl = P.plan->fill[lo];
+    s[t] = nh + nl;
+    __syncthreads();
+    for (int d = 1; d < 1024; d <<= 1) {
+        const int32_t x = t >= d ? s[t - d] : 0;
+        __syncthreads();
+        s[t] += x;
+        __syncthreads();
+    }
+    const int32_t before = s[t] - nh - nl;
+    P.plan->start[hi] = before;
+    P.plan->start[lo] = before + nh;
+    P.plan->fill[hi] = 0;
+    P.plan->fill[lo] = 0;
+    int32_t in_front = 0;
+    if (before < P.head) in_front += nh;
+    if (before + nh < P.head) in_front += nl;
+    if (in_front) atomicAdd(&P.plan->heavy, in_front);
+}
+__global__ void __launch_bounds__(256) k_cost_scatter(CostOrder P) {
+    __shared__ int32_t warp_n[8], base;
+    const int i = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int b = i < P.nsrc ? P.bin(i) : 0;
+    const bool front = i < P.nsrc && P.plan->start[b] < P.head, back = i < P.nsrc && !front;
+    if (front) {
+        const int64_t j = P.plan->start[b] + atomicAdd(&P.plan->fill[b], 1);
+        const int64_t wave = (int64_t)P.warps * P.warp_lanes;  // strided() maps this place to j
+        const int64_t at = j < wave ? (j % P.warps) * P.warp_lanes + j / P.warps : j;
+        P.order[at] = P.sb + i;
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, back);
+    if (lane == 0) warp_n[w] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int32_t n = 0;
+        for (int k = 0; k < 8; ++k) {
+            const int32_t c = warp_n[k];
+            warp_n[k] = n;
+            n += c;
+        }
+        base = P.plan->heavy + (n ? atomicAdd(&P.plan->rest, n) : 0);
+    }
+    __syncthreads();
+    if (back) P.order[base + warp_n[w] + __popc(m & ((1u << lane) - 1u))] = P.sb + i;
+}
+
+// Sources by flag: queue drop, reference-table overflow, watchdog, undefined.
+__global__ void __launch_bounds__(256) k_tally(const int32_t* flags, int32_t n, unsigned long long* out) {
+    int32_t c[4] = {0, 0, 0, 0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int32_t f = flags[i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] += (f >> k) & 1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int32_t s = __reduce_add_sync(0xFFFFFFFFu, c[k]);
+        if ((threadIdx.x & 31) == 0 && s) atomicAdd(&out[k], (unsigned long long)s);
+    }
+}
+
 // ------------------------------------------------------------------ host
 
 namespace {
@@ -760,30 +856,46 @@ svg_build_opts effective_options(const svg_mesh* m, const svg_build_opts& o) {
 }  // namespace
 
 namespace {
-// Flag tallies of a finished build; per-source costs kept on the mesh for
-// the next build's order.
-void record_counts(svg_mesh* m, svg_graph* g, int32_t K, int32_t sb, int32_t se, bool plain, int64_t max_windows) {
+// What a finished build leaves on the device: its counters (acc[0..8]) and, in
+// acc[9..12], the flag tallies.
+constexpr int kAccWords = 13;
+
+// Tally the flags of g behind the counters of `d_acc` and, for a batched
+// build, keep the per-source costs with the mesh for the next build's order;
+// then read the counters (synchronises the library stream).
+void finish_counts(svg_mesh* m, svg_graph* g, int32_t K, int32_t sb, int32_t se, bool plain,
+                   unsigned long long* d_acc, unsigned long long* acc) {
     const int32_t nv = g->nv;
-    svg_build_stats& S = g->stats;
-    std::vector<int32_t> fl((size_t)nv);
-    SVG_CUDA(cudaMemcpy(fl.data(), g->st_flags, sizeof(int32_t) * (size_t)nv, cudaMemcpyDeviceToHost));
+    cudaStream_t st = lib_stream();
+    k_tally<<<std::min((nv + 255) / 256, 592), 256, 0, st>>>(g->st_flags, nv, d_acc + 9);
+    SVG_CUDA(cudaGetLastError());
     if (!plain) {
-        std::vector<int32_t> w((size_t)nv);
-        SVG_CUDA(cudaMemcpy(w.data(), g->st_windows, sizeof(int32_t) * (size_t)nv, cudaMemcpyDeviceToHost));
-        if (m->cost_K != K || (int32_t)m->cost.size() != nv) {
-            m->cost.assign((size_t)nv, 0);
+        m->cost.reserve(sizeof(int32_t) * (size_t)nv);
+        if (m->cost_K != K) {
+            SVG_CUDA(cudaMemsetAsync(m->cost.p, 0, sizeof(int32_t) * (size_t)nv, st));
             m->cost_K = K;
             m->cost_probe = false;
+            m->cost_max = 0;
         }
-        for (int32_t v = sb; v < se; ++v) m->cost[(size_t)v] = w[(size_t)v];
+        SVG_CUDA(cudaMemcpyAsync(m->cost.as<int32_t>() + sb, g->st_windows + sb, sizeof(int32_t) * (size_t)(se - sb),
+                                 cudaMemcpyDeviceToDevice, st));
         if (sb == 0 && se == nv) m->cost_probe = false;
-        m->cost_even = 2 * max_windows * S.sources <= 3 * S.windows;  // largest at most 1.5 times the mean
     }
-    for (int32_t f : fl) {
-        if (f & 1) ++S.queue_drop_sources;
-        if (f & 2) ++S.ref_overflow_sources;
-        if (f & 4) ++S.watchdog_sources;
-        if (f & 8) ++S.undefined_sources;
+    SVG_CUDA(cudaMemcpyAsync(acc, d_acc, sizeof(unsigned long long) * kAccWords, cudaMemcpyDeviceToHost, st));
+    SVG_CUDA(cudaStreamSynchronize(st));
+    svg_build_stats& S = g->stats;
+    S.windows = (int64_t)acc[0];
+    S.windows_generated = (int64_t)acc[1];
+    S.pseudo_sources = (int64_t)acc[2];
+    S.max_win_queue = (int32_t)acc[3];
+    S.max_pseudo_queue = (int32_t)acc[4];
+    S.queue_drop_sources = (int32_t)acc[9];
+    S.ref_overflow_sources = (int32_t)acc[10];
+    S.watchdog_sources = (int32_t)acc[11];
+    S.undefined_sources = (int32_t)acc[12];
+    if (!plain) {
+        m->cost_max = std::max(m->cost_max, (int64_t)acc[5]);
+        m->cost_even = 2 * (int64_t)acc[5] * (se - sb) <= 3 * S.windows;
     }
 }
 
@@ -822,7 +934,7 @@ bool replay_graph(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
     SVG_CUDA(cudaGraphLaunch(bg->exec, st));
     SVG_CUDA(cudaEventRecord(e1, st));
     int32_t retry_n = 0;
-    unsigned long long acc[9] = {0};
+    unsigned long long acc[kAccWords] = {0};
     int64_t nnz = 0;
     SVG_CUDA(cudaMemcpyAsync(&retry_n, bg->d_retry_n, sizeof(retry_n), cudaMemcpyDeviceToHost, st));
     SVG_CUDA(cudaMemcpyAsync(acc, bg->d_acc, sizeof(acc), cudaMemcpyDeviceToHost, st));
@@ -844,11 +956,6 @@ bool replay_graph(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
     S.ms_ich = ms_ich;
     S.ms_emit = ms_emit;
     S.ms_total = ms;
-    S.windows = (int64_t)acc[0];
-    S.windows_generated = (int64_t)acc[1];
-    S.pseudo_sources = (int64_t)acc[2];
-    S.max_win_queue = (int32_t)acc[3];
-    S.max_pseudo_queue = (int32_t)acc[4];
     S.edges = nnz;
     S.sources = bg->nsrc;
     S.launches = (SVG_SPLIT_TRACE && bg->opts.with_paths) ? 4 : 3;  // k_ich_batched, the offsets scan,
@@ -857,7 +964,7 @@ bool replay_graph(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
     S.coop_sources = bg->coop_n;
     S.coop_warps = bg->coop_warps;
     S.graph_replayed = 1;
-    record_counts(m, g, o.K, bg->sb, bg->se, false, (int64_t)acc[5]);
+    finish_counts(m, g, o.K, bg->sb, bg->se, false, bg->d_acc, acc);
     return true;
 }
 
@@ -1040,7 +1147,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     }
     if (!plain && o.heavy_first == 2 && nsrc > full_lanes && K >= 160 &&
         3 * (int64_t)nsrc <= 8 * (int64_t)full_lanes &&
-        !(m->cost_K == K && (int32_t)m->cost.size() == nv)) {
+        m->cost_K != K) {
         svg_build_opts po = o;
         po.K = K / 10;
         po.heavy_first = 0;
@@ -1054,10 +1161,8 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
             throw;
         }
         free_graph_device(&pg);
-        if ((int32_t)m->cost.size() == nv) {
-            m->cost_K = K;  // the probe's costs stand in for K's
-            m->cost_probe = true;
-        }
+        m->cost_K = K;  // the probe's costs stand in for K's
+        m->cost_probe = true;
     }
 
     int dev = 0;
@@ -1099,9 +1204,14 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     C.vlimit = lay.vlimit;
     C.slimit = (int32_t)(((int64_t)3 << lay.scap_log2) / 4);
 
-    size_t freeb = 0, totalb = 0;
-    SVG_CUDA(cudaMemGetInfo(&freeb, &totalb));
-    int64_t budget = o.hbm_budget > 0 ? o.hbm_budget : (int64_t)((double)freeb * 0.5);
+    // whether scratch of this size, for which `held` bytes are there already, is within the budget
+    auto fits = [&](size_t bytes, size_t held) {
+        if (o.hbm_budget > 0) return (int64_t)bytes <= o.hbm_budget;
+        if (bytes <= held) return true;  // nothing to allocate: the query costs more than a small build's launches
+        size_t freeb = 0, totalb = 0;
+        SVG_CUDA(cudaMemGetInfo(&freeb, &totalb));
+        return (double)bytes <= 0.5 * (double)freeb;
+    };
 
     int tpb = o.threads_per_block > 0 ? o.threads_per_block : 128;
     if (tpb % 32 != 0 || tpb > 128) throw SvgError{SVG_ERR_ARG, "threads_per_block must be a multiple of 32, <= 128"};
@@ -1138,8 +1248,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         // field K = 500 438 / 411 ms, but K = 100 26.2 / 28.7 ms and 120K
         // K = 200 134 / 141 ms.
         const int64_t warps = (int64_t)blocks * (tpb / 32);
-        const bool costs = m->cost_K == K && (int32_t)m->cost.size() == nv;
-        const bool equal = K >= 300 || (costs && m->cost_even);
+        const bool equal = K >= 300 || (m->cost_K == K && m->cost_even);
         const int64_t waves = equal ? std::max<int64_t>(1, (nsrc + 32 * warps - 1) / (32 * warps)) : 1;
         warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps * waves - 1) / (warps * waves)));
         const int64_t per_block = (int64_t)(tpb / 32) * warp_lanes;
@@ -1147,11 +1256,11 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     }
     const int block_lanes = plain ? tpb : (tpb / 32) * warp_lanes;
     lay.lanes = blocks * block_lanes;
-    while (blocks > 1 && (int64_t)(lane_bytes(lay) * lay.lanes) > budget) {
+    while (blocks > 1 && !fits(lane_bytes(lay) * lay.lanes, g_arena[0].buf.bytes)) {
         blocks = std::max(1, blocks / 2);
         lay.lanes = blocks * block_lanes;
     }
-    if ((int64_t)(lane_bytes(lay) * lay.lanes) > budget)
+    if (!fits(lane_bytes(lay) * lay.lanes, g_arena[0].buf.bytes))
         throw SvgError{SVG_ERR_NOMEM, "HBM budget too small for one block of build lanes"};
 
     carve(g_arena[0], lay, C, st);
@@ -1168,25 +1277,45 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     bool ordered = false;
     const bool one_wave = nsrc <= lay.lanes;
     const int32_t wave_warps = plain ? 0 : std::min(nsrc, lay.lanes) / warp_lanes;
-    if (!plain && o.heavy_first && m->cost_K == K && (int32_t)m->cost.size() == nv && nsrc > 0 &&
-        (!one_wave || o.coop_sources != 0)) {
-        // The heaviest sources, two per lane, go first (they would otherwise
-        // set the tail); the rest keep vertex order, so that the sources in
-        // flight together stay neighbours on the mesh and share its lines in L2
-        // (full heaviest-first order is 3 % slower on the 750K torus, vertex
-        // order 13 % slower on the 72.9K height field).
-        std::vector<int32_t> ord((size_t)nsrc);
+    // The heaviest sources, two per lane, go first (they would otherwise
+    // set the tail); the rest keep vertex order, so that the sources in
+    // flight together stay neighbours on the mesh and share its lines in L2
+    // (full heaviest-first order is 3 % slower on the 750K torus, vertex
+    // order 13 % slower on the 72.9K height field).
+    const int64_t head = std::min<int64_t>(nsrc, (int64_t)lay.lanes * o.heavy_waves);
+    const bool by_cost = !plain && o.heavy_first && m->cost_K == K && nsrc > 0;
+    DevBuf b_plan;
+    if (by_cost && o.coop_sources == 0 && !one_wave) {
+        CostOrder P{};
+        P.cost = m->cost.as<int32_t>();
+        P.sb = sb;
+        P.nsrc = nsrc;
+        P.head = (int32_t)head;
+        while ((m->cost_max >> P.shift) >= kCostBins) ++P.shift;
+        P.warps = wave_warps;
+        P.warp_lanes = warp_lanes;
+        b_plan.reserve(sizeof(CostPlan));
+        P.plan = b_plan.as<CostPlan>();
+        P.order = d_order;
+        SVG_CUDA(cudaMemsetAsync(P.plan, 0, sizeof(CostPlan), st));
+        k_cost_hist<<<std::min((nsrc + 255) / 256, 2 * prop.multiProcessorCount), 256, 0, st>>>(P);
+        k_cost_plan<<<1, 1024, 0, st>>>(P);
+        k_cost_scatter<<<(nsrc + 255) / 256, 256, 0, st>>>(P);
+        SVG_CUDA(cudaGetLastError());
+        ordered = true;
+    } else if (by_cost && o.coop_sources != 0) {
+        // the cooperative warps take their sources from the front, in cost order
+        std::vector<int32_t> cost((size_t)nv), ord((size_t)nsrc);
+        SVG_CUDA(cudaMemcpyAsync(cost.data(), m->cost.p, sizeof(int32_t) * (size_t)nv, cudaMemcpyDeviceToHost, st));
+        SVG_CUDA(cudaStreamSynchronize(st));
         for (int32_t i = 0; i < nsrc; ++i) ord[(size_t)i] = sb + i;
-        const int64_t head = std::min<int64_t>(nsrc, (int64_t)lay.lanes * o.heavy_waves);
         std::vector<int32_t> byc(ord);
         std::stable_sort(byc.begin(), byc.end(),
-                         [&](int32_t a, int32_t b) { return m->cost[(size_t)a] > m->cost[(size_t)b]; });
+                         [&](int32_t a, int32_t b) { return cost[(size_t)a] > cost[(size_t)b]; });
         std::vector<char> taken((size_t)nsrc, 0);
-        // the cooperative warps take their sources from the front, in cost order
-        const int32_t stride_warps = o.coop_sources != 0 ? 0 : wave_warps;
         for (int64_t i = 0; i < head; ++i) {
-            ord[(size_t)i] = byc[(size_t)strided(i, stride_warps, warp_lanes)];
-            taken[(size_t)ord[(size_t)i] - (size_t)sb] = 1;
+            ord[(size_t)i] = byc[(size_t)i];
+            taken[(size_t)(byc[(size_t)i] - sb)] = 1;
         }
         int64_t k = head;
         for (int32_t i = 0; i < nsrc; ++i)
@@ -1201,13 +1330,13 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         // 200 hold 27 of K=500's top 200), and the tail adoption covers them.
         if (o.coop_sources > 0 || (o.coop_sources < 0 && !m->cost_probe)) {
             double total = 0.0;
-            for (int32_t i = 0; i < nsrc; ++i) total += (double)m->cost[(size_t)(sb + i)];
+            for (int32_t i = 0; i < nsrc; ++i) total += (double)cost[(size_t)(sb + i)];
             const double share = total / (double)lay.lanes;
             int64_t n = 0;
             if (o.coop_sources > 0) {
                 n = std::min<int64_t>(o.coop_sources, nsrc);
             } else {
-                while (n < head && (double)m->cost[(size_t)ord[(size_t)n]] >= share) ++n;
+                while (n < head && (double)cost[(size_t)ord[(size_t)n]] >= share) ++n;
                 n = std::min<int64_t>(n, lay.lanes / 64);
             }
             const int64_t warps = (int64_t)blocks * (tpb / 32);
@@ -1345,7 +1474,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                 const int wl2 = (int)std::min<int64_t>(32, ((int64_t)retry_n + 2 * bl2 - 1) / (2 * bl2));
                 bl2 = (int)std::min<int64_t>(bl2, ((int64_t)retry_n + 2 * wl2 - 1) / (2 * wl2));
                 l2.lanes = bl2 * 2 * wl2;
-                while (bl2 > 1 && (int64_t)(lane_bytes(l2) * l2.lanes) > budget) {
+                while (bl2 > 1 && !fits(lane_bytes(l2) * l2.lanes, g_arena[1].buf.bytes)) {
                     bl2 = std::max(1, bl2 / 2);
                     l2.lanes = bl2 * 2 * wl2;
                 }
@@ -1438,10 +1567,9 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     }
     SVG_CUDA(cudaGetLastError());
     SVG_CUDA(cudaEventRecord(ev[3], st));
-    SVG_CUDA(cudaStreamSynchronize(st));
-
-    unsigned long long acc[8] = {0};
-    SVG_CUDA(cudaMemcpy(acc, d_acc, sizeof(acc), cudaMemcpyDeviceToHost));
+    g->stats = svg_build_stats{};
+    unsigned long long acc[kAccWords] = {0};
+    finish_counts(m, g, K, sb, se, plain, d_acc, acc);
     float t01 = 0, t23 = 0, t03 = 0;
     SVG_CUDA(cudaEventElapsedTime(&t01, ev[0], ev[1]));
     SVG_CUDA(cudaEventElapsedTime(&t23, ev[2], ev[3]));
@@ -1449,15 +1577,9 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     for (auto& e : ev) cudaEventDestroy(e);
 
     svg_build_stats& S = g->stats;
-    S = svg_build_stats{};
     S.ms_ich = t01;
     S.ms_emit = t23;
     S.ms_total = t01 + t23;  // excludes the host-side CSR allocation between the phases
-    S.windows = (int64_t)acc[0];
-    S.windows_generated = (int64_t)acc[1];
-    S.pseudo_sources = (int64_t)acc[2];
-    S.max_win_queue = (int32_t)acc[3];
-    S.max_pseudo_queue = (int32_t)acc[4];
     S.edges = nnz;
     S.sources = nsrc;
     S.retried_sources = retry_n;
@@ -1466,7 +1588,6 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     S.coop_sources = coop_n;
     S.coop_warps = coop_warps;
     (void)t03;
-    record_counts(m, g, K, sb, se, plain, (int64_t)acc[5]);
     if (o.graph && !plain && nsrc > 0 && retry_n == 0 && cap_attempts == 0) {
         CapturePlan P;
         P.C = C;

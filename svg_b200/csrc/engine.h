@@ -75,10 +75,11 @@ struct svg_mesh {
     svgb::HostMesh h;
     svgb::MeshDev d;
     // Per-source cost (windows propagated) measured by the last batched build
-    // at K = cost_K: the next build at the same K orders its work queue
-    // heaviest first (longest-processing-time first).
+    // at K = cost_K, on the device: the next build at the same K orders its
+    // work queue heaviest first (longest-processing-time first).
     int32_t cost_K = 0;
-    std::vector<int32_t> cost;
+    svgb::DevBuf cost;
+    int64_t cost_max = 0;  // the largest of them
     // the costs are a K/10 probe build's stand-in, not a build at cost_K
     bool cost_probe = false;
     // the costliest source of that build took at most 1.5 times the mean

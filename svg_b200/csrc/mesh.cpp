@@ -136,6 +136,7 @@ std::string build_host_mesh(int32_t nv, const double* pos, int32_t nf, const int
             h.v0 = a;
             h.v1 = c;
             h.twin = -1;
+            h.vflags = 0;  // filled in on the device, from the vertex records
             h.corner = 0.0;
             const double* pa = &pos[3 * (size_t)a];
             const double* pb = &pos[3 * (size_t)c];
@@ -215,11 +216,6 @@ std::string build_host_mesh(int32_t nv, const double* pos, int32_t nf, const int
         if (m.angle[v] > 2.0 * kPi) fl |= kVertSaddleGT;     // saddle test of PropagateWindow
         m.vr[v].flags = fl;
     }
-    auto copy_flags = [&](int64_t b, int64_t e_end) {
-        for (int64_t e = b; e < e_end; ++e) m.he[e].vflags = m.vr[m.he[e].v1].flags;
-    };
-    if (E < 1 << 19) copy_flags(0, E);  // starting the threads would take longer than the loop
-    else parallel_for(E, copy_flags);
     return std::string();
 }
 
