@@ -128,6 +128,7 @@ struct svg_qctx {
     svgb::DevBuf buf;
     uint32_t* stamps = nullptr;
     int32_t* head = nullptr;
+    void* ctl = nullptr;  // per slot: counters and barrier of the grid form
     int cluster = 0;  // blocks per query: a cluster of them, or 0 for one block (the plain form)
     bool adaptive = false;  // large batches switch to 8-block clusters
 };

@@ -19,6 +19,7 @@
 // Per-slot stamp arrays replace clearing: a stamp is never reused.
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -46,6 +47,8 @@ struct alignas(16) DS {
     long long s;           // source id (-1 = none)
 };
 
+struct QCtl;
+
 struct QParams {
     const int64_t* off;
     const int32_t* adj;
@@ -68,9 +71,19 @@ struct QParams {
     char* scratch;
     size_t slot_bytes;
     uint32_t* slot_stamp;  // per slot
-    int32_t* head;
+    int32_t* head;         // kHead*
     int64_t list_cap;      // far list capacity (entries)
+    // grid form: blocks per query, and per query slot its counters and barrier
+    int32_t group;
+    QCtl* ctl;
+    int32_t fallback;      // cluster form: run only if the grid form before it did not
 };
+// Words of QParams::head; the first four are zeroed before every launch.
+//   kHeadNext    next query
+//   kHeadState   grid form: 0 gathering, 1 every block is there, 2 given up
+//   kHeadJoined  blocks there
+//   kHeadBroken  a barrier ran out: the context's slots are unusable
+enum { kHeadNext = 0, kHeadState = 1, kHeadJoined = 2, kHeadBroken = 8, kHeadZeroed = 4 };
 
 __device__ __forceinline__ double hdist(const double* pos, int a, int b) {
     double dx = pos[3 * a] - pos[3 * b], dy = pos[3 * a + 1] - pos[3 * b + 1], dz = pos[3 * a + 2] - pos[3 * b + 2];
@@ -340,11 +353,13 @@ __global__ void __launch_bounds__(kQThreads) k_query(QParams P) {
 }
 
 // ---------------------------------------------------------------------------
-// Cluster form: one query per thread-block cluster (8 or 16 SMs).  A batch runs
-// only as many queries at once as there are clusters, so each query's
-// distance and flag arrays stay in L2 while many SMs expand its frontier;
-// per-block query concurrency (the single-block form above) thrashes L2 on
-// large graphs.  The search is the same near-far label-correcting one, with:
+// Team forms: one query per team of blocks, a thread-block cluster (8 or 16
+// blocks) or, for a few whole-graph searches, an equal share of every block
+// the GPU holds.  A batch runs only as many queries at once as there are
+// teams, so each query's distance and flag arrays stay in L2 while many SMs
+// expand its frontier; per-block query concurrency (the single-block form
+// above) thrashes L2 on large graphs.  The search is the same near-far
+// label-correcting one, with (cluster form):
 //   * cluster barriers (hardware, no spinning) in place of __syncthreads;
 //   * the phase counters in the first block's shared memory, reached by the
 //     others through distributed shared memory, appended to with one atomic
@@ -373,6 +388,8 @@ struct QCtl {
     int q;                       // query being served
     int init_far;                // far list length after the sources
     uint32_t stamp;              // slot stamp at the query's start
+    unsigned arrived;            // grid form: barrier arrivals since the launch
+    int failed;                  // grid form: a barrier wait ran out
 };
 
 // Append the lanes with pred set to a list whose length is *counter (which may
@@ -405,31 +422,189 @@ __device__ __forceinline__ DS ld_ds(const DS* p) {
     return r;
 }
 
-template <bool kSSSD, bool kSrc>
-__global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParams P) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
+// The blocks that serve one query together.
+//   ClusterTeam  a thread-block cluster: hardware barrier, counters in the
+//                first block's shared memory.
+//   GridTeam     any number of blocks of a launch no larger than the GPU holds:
+//                counters in global memory and a barrier on one of them.  The
+//                blocks of the launch first gather (join): where other streams
+//                hold the GPU and some block has not come after a few
+//                milliseconds, all leave again before any query is begun, and
+//                the cluster form enqueued behind them serves the batch.  Once
+//                all are there they stay, so a barrier's wait is short; it gives
+//                up after kBarrierSpins looks (seconds), and the launch's
+//                unfinished queries and all later ones of the context report -1.
+struct ClusterTeam {
+    QCtl* ctl;
+    int size, rank, slot;
+    __device__ ClusterTeam(const QParams&, QCtl* s_ctl) {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cl = cg::this_cluster();
+        ctl = cl.map_shared_rank(s_ctl, 0);
+        size = (int)cl.num_blocks();
+        rank = (int)cl.block_rank();
+        slot = (int)blockIdx.x / size;
+    }
+    __device__ bool join(const QParams& P) {
+        return !P.fallback || *(volatile int32_t*)&P.head[kHeadState] == 2;
+    }
+    __device__ bool sync() {
+        cooperative_groups::this_cluster().sync();
+        return true;
+    }
+};
+constexpr int kBarrierSpins = 1 << 22;
+#ifndef SVG_JOIN_SPINS
+#define SVG_JOIN_SPINS (1 << 14)
+#endif
+struct GridTeam {
+    QCtl* ctl;
+    int size, rank, slot;
+    unsigned phase;
+    __device__ GridTeam(const QParams& P, QCtl*) {
+        size = P.group;
+        slot = (int)blockIdx.x / size;
+        rank = (int)blockIdx.x % size;
+        ctl = P.ctl + slot;
+        phase = 0;
+    }
+    __device__ bool join(const QParams& P) {
+        int s = 0;
+        if (threadIdx.x == 0) {
+            int32_t* state = &P.head[kHeadState];
+            if (atomicAdd(&P.head[kHeadJoined], 1) + 1 == (int)gridDim.x) atomicCAS(state, 0, 1);
+            for (int spins = 0; (s = *(volatile int32_t*)state) == 0; ++spins)
+                if (spins >= SVG_JOIN_SPINS) {
+                    s = atomicCAS(state, 0, 2);  // one word decides for all blocks
+                    if (s == 0) s = 2;
+                    break;
+                }
+        }
+        return __syncthreads_or(s == 1) != 0;
+    }
+    // false: some block of the team never arrived; every block leaves
+    __device__ bool sync() {
+        phase += (unsigned)size;
+        __syncthreads();
+        int ok = 1;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(&ctl->arrived, 1u);
+            volatile unsigned* a = &ctl->arrived;
+            int spins = 0;
+            while ((int)(*a - phase) < 0 && ++spins < kBarrierSpins) {
+            }
+            if (spins >= kBarrierSpins) atomicExch(&ctl->failed, 1);
+            __threadfence();
+            ok = *(volatile int*)&ctl->failed ? 0 : 1;
+        }
+        return __syncthreads_and(ok) != 0;
+    }
+};
+
+// Block-local staging of the lists a grid team appends to: one global atomic
+// per block and round instead of one per warp and edge batch (thousands of
+// warps on one counter would queue up).  An entry that finds it full goes to
+// the global list directly.
+constexpr int kStage = 1024;
+struct Stage {
+    int32_t v[kStage];
+    int n;
+};
+__device__ __forceinline__ void stage_put(Stage& S, bool pred, int v, int* counter, int32_t* list, int64_t cap,
+                                          int lane) {
+    const unsigned m = __ballot_sync(0xffffffffu, pred);
+    if (m == 0) return;
+    const int first = __ffs(m) - 1, k = __popc(m);
+    int base = 0, at = 0;
+    if (lane == first) {
+        base = atomicAdd(&S.n, k);
+        // what does not fit is appended at once
+        const int over = min(k, max(0, base + k - kStage));
+        at = over ? atomicAdd(counter, over) : 0;
+    }
+    base = __shfl_sync(0xffffffffu, base, first);
+    at = __shfl_sync(0xffffffffu, at, first);
+    if (pred) {
+        const int i = base + __popc(m & ((1u << lane) - 1u));
+        if (i < kStage) S.v[i] = v;
+        else if (const int64_t j = at + (i - max(base, kStage)); j < cap) list[j] = v;
+    }
+}
+// Every thread of the block calls it, between two barriers of the team.
+__device__ __forceinline__ void stage_flush(Stage& S, int* counter, int32_t* list, int64_t cap, int* s_base) {
+    __syncthreads();
+    const int n = min(S.n, kStage);
+    if (n) {  // uniform: S.n is not written between the two __syncthreads
+        if (threadIdx.x == 0) *s_base = atomicAdd(counter, n);
+        __syncthreads();
+        const int base = *s_base;
+        for (int i = threadIdx.x; i < n; i += blockDim.x)
+            if (base + (int64_t)i < cap) list[base + i] = S.v[i];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) S.n = 0;
+}
+
+// One query at a time per team (see the comment at the top of this section).
+// (Gathering MSAD distances from an 8-byte copy beside the {distance, source}
+// pairs halves the gathered sectors but adds a pair load and an atomic to every
+// improvement: 6 % slower on the 750K torus.)
+template <bool kSSSD, bool kSrc, class Team>
+__global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P) {
+    constexpr bool kStaged = !std::is_same<Team, ClusterTeam>::value;
     __shared__ QCtl s_ctl;
-    QCtl* ctl = cl.map_shared_rank(&s_ctl, 0);
-    const int csize = (int)cl.num_blocks();
-    const int crank = (int)cl.block_rank();
-    const int slot = (int)blockIdx.x / csize;
-    Slot S = carve_slot(P, slot);
+    __shared__ Stage s_near, s_far;
+    __shared__ int s_base;
+    Team team(P, &s_ctl);
+    QCtl* ctl = team.ctl;
+    Slot S = carve_slot(P, team.slot);
     const int tid = threadIdx.x, lane = tid & 31;
-    const int nthr = csize * kCThreads, gtid = crank * kCThreads + tid;
+    const int nthr = team.size * kCThreads, gtid = team.rank * kCThreads + tid;
     const int gwarp = gtid >> 5, nwarps = nthr >> 5;
-    const bool leader = crank == 0 && tid == 0;
+    const bool leader = team.rank == 0 && tid == 0;
     const long long round_cap = 64LL * ((long long)P.nv + 16);
+    if (kStaged && tid == 0) s_near.n = s_far.n = 0;
+    // append v where pred, to the list whose length is *counter
+    auto put = [&](Stage& st, bool pred, int v, int* counter, int32_t* list, int64_t cap) {
+        if constexpr (kStaged) {
+            stage_put(st, pred, v, counter, list, cap, lane);
+        } else {
+            const int p = warp_append(pred, counter, lane);
+            if (p >= 0 && p < cap) list[p] = v;
+        }
+    };
+
+    // a barrier ran out in this launch or an earlier one: -1 for query q and
+    // all that no team has taken
+    auto give_up = [&](int q) {
+        if (tid == 0) atomicExch(&P.head[kHeadBroken], 1);
+        for (;;) {
+            if (q >= 0 && kSSSD && tid == 0) P.out[q] = -1.0;
+            if (q >= 0 && !kSSSD)
+                for (int v = tid; v < P.nv; v += kCThreads) P.out_dist[(size_t)q * P.nv + v] = -1.0;
+            __syncthreads();
+            if (tid == 0) s_base = atomicAdd(&P.head[kHeadNext], 1);
+            __syncthreads();
+            q = s_base;
+            if (q >= P.n) return;
+        }
+    };
+    if (!team.join(P)) return;
+    if (*(volatile int32_t*)&P.head[kHeadBroken]) {
+        give_up(-1);
+        return;
+    }
 
     for (;;) {
         if (leader) {
-            ctl->q = atomicAdd(P.head, 1);
-            ctl->stamp = P.slot_stamp[slot];
+            ctl->q = atomicAdd(&P.head[kHeadNext], 1);
+            ctl->stamp = P.slot_stamp[team.slot];
         }
-        cl.sync();
-        const int q = ctl->q;
-        uint32_t stamp = ctl->stamp;
-        cl.sync();  // q and stamp read everywhere before the leader moves on (or any block leaves)
+        if (!team.sync()) return give_up(-1);
+        const int q = *(volatile int*)&ctl->q;
+        uint32_t stamp = *(volatile uint32_t*)&ctl->stamp;
+        if (!team.sync()) return give_up(q < P.n ? q : -1);  // q and stamp read everywhere before the leader moves on (or any block leaves)
         if (q >= P.n) break;
         const int tgt = kSSSD ? P.t[q] : -1;
 
@@ -451,7 +626,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                 S.ds[v] = z;
             }
         }
-        cl.sync();
+        if (!team.sync()) return give_up(q);
         stamp += 1;
         const uint32_t fst = stamp;
         if (leader) {
@@ -482,8 +657,8 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
             }
             ctl->init_far = nf;
         }
-        cl.sync();
-        int farN = ctl->init_far;
+        if (!team.sync()) return give_up(q);
+        int farN = *(volatile int*)&ctl->init_far;
         int32_t *far = S.far, *far2 = S.far2, *near = S.near, *next = S.next;
         long long rounds = 0;
         int o = 0, gr = 0;
@@ -513,9 +688,9 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                 ctl->nearA[nb] = 0;
                 ctl->farB[nb] = 0;
             }
-            cl.sync();
+            if (!team.sync()) return give_up(q);
             if (farN == 0) break;
-            const double fmin = as_d(ctl->fmin[ob]);
+            const double fmin = as_d(*(volatile unsigned long long*)&ctl->fmin[ob]);
             if (kSSSD && as_d(__ldcg(&S.dist[tgt])) <= fmin) break;  // no waiting path can beat the target
             const double thr = fmin + P.delta;
             stamp += 2;
@@ -532,16 +707,18 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                     if (f < thr) to_near = atomicExch(&S.nflag[v], nst) != nst;
                     else to_far = atomicExch(&S.fflag[v], fst2) != fst2;
                 }
-                int p = warp_append(to_near, &ctl->nearA[ob], lane);
-                if (p >= 0) near[p] = v;
-                p = warp_append(to_far, &ctl->farB[ob], lane);
-                if (p >= 0 && p < P.list_cap) far2[p] = v;
+                put(s_near, to_near, v, &ctl->nearA[ob], near, P.nv);
+                put(s_far, to_far, v, &ctl->farB[ob], far2, P.list_cap);
             }
-            cl.sync();
+            if constexpr (kStaged) {
+                stage_flush(s_near, &ctl->nearA[ob], near, P.nv, &s_base);
+                stage_flush(s_far, &ctl->farB[ob], far2, P.list_cap, &s_base);
+            }
+            if (!team.sync()) return give_up(q);
             {
                 int32_t* t = far; far = far2; far2 = t;
             }
-            int nearN = ctl->nearA[ob];
+            int nearN = *(volatile int*)&ctl->nearA[ob];
 
             // drain the near frontier: one warp per vertex, lanes over its edges
             while (nearN > 0) {
@@ -578,7 +755,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                         long long curs[kQUnroll];
 #pragma unroll
                         for (int j = 0; j < kQUnroll; ++j) {
-                            curd[j] = kInfBits;
+                            curd[j] = 0ull;
                             curs[j] = -1;
                             if (wv[j] < 0) continue;
                             if (kSSSD) {
@@ -593,7 +770,9 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                         for (int j = 0; j < kQUnroll; ++j) {
                             const int w = wv[j];
                             bool to_next = false, to_far = false, to_touch = false;
-                            if (w >= 0 && nd[j] < as_d(curd[j])) {
+                            const bool maybe = w >= 0 && nd[j] < as_d(curd[j]);
+                            if (!__any_sync(0xffffffffu, maybe)) continue;
+                            if (maybe) {
                                 bool improved = false;
                                 if (kSSSD) {
                                     const unsigned long long old = atomicMin(&S.dist[w], as_b(nd[j]));
@@ -621,27 +800,28 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                                     else to_far = atomicExch(&S.fflag[w], fst2) != fst2;
                                 }
                             }
-                            int p;
                             if (kSSSD) {
-                                p = warp_append(to_touch, &ctl->touch, lane);
+                                const int p = warp_append(to_touch, &ctl->touch, lane);
                                 if (p >= 0) S.touched[p] = w;
                             }
-                            p = warp_append(to_next, &ctl->nextX[gb], lane);
-                            if (p >= 0) next[p] = w;
-                            p = warp_append(to_far, &ctl->farB[ob], lane);
-                            if (p >= 0 && p < P.list_cap) far[p] = w;
+                            put(s_near, to_next, w, &ctl->nextX[gb], next, P.nv);
+                            put(s_far, to_far, w, &ctl->farB[ob], far, P.list_cap);
                         }
                     }
                 }
-                cl.sync();
-                nearN = ctl->nextX[gb];
+                if constexpr (kStaged) {
+                    stage_flush(s_near, &ctl->nextX[gb], next, P.nv, &s_base);
+                    stage_flush(s_far, &ctl->farB[ob], far, P.list_cap, &s_base);
+                }
+                if (!team.sync()) return give_up(q);
+                nearN = *(volatile int*)&ctl->nextX[gb];
                 {
                     int32_t* t = near; near = next; next = t;
                 }
                 ++gr;
             }
             if (over) break;
-            farN = ctl->farB[ob];
+            farN = *(volatile int*)&ctl->farB[ob];
             ++o;
         }
 
@@ -652,8 +832,8 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                 const unsigned long long dt = __ldcg(&S.dist[tgt]);
                 P.out[q] = ovf ? -1.0 : (dt == kInfBits ? DBL_MAX : as_d(dt));
             }
-            cl.sync();  // the target's distance is read before the reset below
-            const int tn = ctl->touch;
+            if (!team.sync()) return give_up(q);  // the target's distance is read before the reset below
+            const int tn = *(volatile int*)&ctl->touch;
             for (int i = gtid; i < tn; i += nthr) S.dist[__ldcg(&S.touched[i])] = kInfBits;
         } else {
             double* od = P.out_dist + (size_t)q * P.nv;
@@ -664,8 +844,8 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_cluster(QParam
                 if (kSrc) os[v] = (int32_t)z.s;
             }
         }
-        if (leader) P.slot_stamp[slot] = stamp;
-        cl.sync();
+        if (leader) P.slot_stamp[team.slot] = stamp;
+        if (!team.sync()) return give_up(q);
     }
 }
 
@@ -790,9 +970,9 @@ cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* at, int nclusters, int cs
 void allow_large_clusters() {
     static bool done = false;
     if (done) return;
-    SVG_CUDA(cudaFuncSetAttribute(k_query_cluster<true, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    SVG_CUDA(cudaFuncSetAttribute(k_query_cluster<false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    SVG_CUDA(cudaFuncSetAttribute(k_query_cluster<false, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SVG_CUDA(cudaFuncSetAttribute(k_query_team<true, false, ClusterTeam>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SVG_CUDA(cudaFuncSetAttribute(k_query_team<false, true, ClusterTeam>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SVG_CUDA(cudaFuncSetAttribute(k_query_team<false, false, ClusterTeam>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     done = true;
 }
 
@@ -801,7 +981,37 @@ void launch_cluster(const QParams& P, int nclusters, int csize, cudaStream_t st)
     allow_large_clusters();
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = cluster_config<A, B>(&at, nclusters, csize, st);
-    SVG_CUDA(cudaLaunchKernelEx(&cfg, k_query_cluster<A, B>, P));
+    SVG_CUDA(cudaLaunchKernelEx(&cfg, k_query_team<A, B, ClusterTeam>, P));
+}
+
+// Queries a grid-form launch serves at most, one team of blocks each.  Measured
+// (kernel time, clusters against teams): one MSAD on the 750K torus at K = 100
+// 8.85 / 1.38 ms, 4 of them 9.5 / 3.2, 16 19.6 / 11.3, 32 22.4 / 21.8; on the
+// 73K height field at K = 200 1 1.60 / 0.55 ms, 16 2.8 / 1.7, 32 3.1 / 3.2; on
+// a 30K graph 1 0.69 / 0.46 ms, 4 0.73 / 0.53, 16 1.05 / 0.81, 32 1.10 / 1.12.
+// A single-pair search touches too few vertices a round for that: a cluster
+// of 16 took 0.77 ms on the 750K torus, teams of 37 to 148 blocks 0.71-0.83,
+// and 0.18 against 0.24 ms on a 30K graph.
+constexpr int kGridQueries = 16;
+
+// Blocks of the grid form that run at once.
+int grid_blocks() {
+    static int n = 0;
+    if (n <= 0) {
+        int dev = 0, sms = 0, per_sm = 0;
+        SVG_CUDA(cudaGetDevice(&dev));
+        SVG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        SVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_query_team<false, true, GridTeam>, kCThreads, 0));
+        n = std::max(1, per_sm) * sms;
+    }
+    return n;
+}
+
+template <bool kSrc>
+void launch_grid(QParams& P, int teams, int group, cudaStream_t st) {
+    P.group = group;
+    SVG_CUDA(cudaMemsetAsync(P.ctl, 0, sizeof(QCtl) * (size_t)teams, st));
+    k_query_team<false, kSrc, GridTeam><<<teams * group, kCThreads, 0, st>>>(P);
 }
 
 int max_active_clusters(int csize) {
@@ -809,7 +1019,7 @@ int max_active_clusters(int csize) {
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = cluster_config<false, true>(&at, 1, csize, nullptr);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_query_cluster<false, true>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_query_team<false, true, ClusterTeam>, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -868,7 +1078,8 @@ svg_qctx* qctx_create(svg_graph* g, int slots, cudaStream_t st, int cluster) {
     c->list_cap = 2 * (int64_t)V + 64;
     c->slot_bytes = al256(8 * V) + al256(16 * V) + 4 * al256(4 * V) + 2 * al256(4 * (size_t)c->list_cap) + al256(4 * V);
     const size_t body = al256((size_t)c->slots * c->slot_bytes);
-    const size_t need = body + al256(sizeof(uint32_t) * (size_t)c->slots) + 256;
+    const size_t ctl_at = body + al256(sizeof(uint32_t) * (size_t)c->slots) + 256;
+    const size_t need = ctl_at + sizeof(QCtl) * (size_t)c->slots;
     try {
         c->buf.reserve(need);
     } catch (...) {
@@ -878,6 +1089,7 @@ svg_qctx* qctx_create(svg_graph* g, int slots, cudaStream_t st, int cluster) {
     char* base = c->buf.as<char>();
     c->stamps = reinterpret_cast<uint32_t*>(base + body);
     c->head = reinterpret_cast<int32_t*>(base + body + al256(sizeof(uint32_t) * (size_t)c->slots));
+    c->ctl = base + ctl_at;
     SVG_CUDA(cudaMemsetAsync(base, 0, need, st));  // stamps and flags start at 0
     for (int sl = 0; sl < c->slots; ++sl)          // SSSD distances start at +inf
         k_fill<<<64, 256, 0, st>>>(reinterpret_cast<unsigned long long*>(base + (size_t)sl * c->slot_bytes), V,
@@ -896,6 +1108,7 @@ void fill_params(svg_qctx* c, QParams& P) {
     P.slot_bytes = c->slot_bytes;
     P.slot_stamp = c->stamps;
     P.head = c->head;
+    P.ctl = reinterpret_cast<QCtl*>(c->ctl);
     P.list_cap = c->list_cap;
     P.off = g->off;
     P.adj = g->adj;
@@ -914,7 +1127,7 @@ void qctx_sssd(svg_qctx* c, int32_t n, const int32_t* d_s, const int32_t* d_t, d
     P.s = d_s;
     P.t = d_t;
     P.out = d_dist;
-    SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t), st));
+    SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t) * kHeadZeroed, st));
     if (c->cluster > 0) {
         const int cs = call_cluster(c, n);
         launch_cluster<true, false>(P, std::min(std::min(n, c->slots), query_cluster_slots(cs)), cs, st);
@@ -934,8 +1147,22 @@ void qctx_msad(svg_qctx* c, int32_t n, const int64_t* d_off, const int32_t* d_sr
     P.weights = d_w;
     P.out_dist = d_dist;
     P.out_src = d_src_id;
-    SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t), st));
+    SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t) * kHeadZeroed, st));
     const int nb = std::min(n, c->slots);
+    if (c->adaptive && n <= std::min(kGridQueries, c->slots)) {
+        // Few queries: every block of the GPU serves them, an equal team each.
+        // The fewer the phases, the fewer the barriers: with teams this wide
+        // the extra relaxations of eight-fold buckets (1.27 V instead of 1.10 V
+        // on the 750K torus, in 66 phases instead of 179) cost less than they
+        // save (one MSAD 1.97 ms with two-fold buckets, 1.38 with eight-fold).
+        const int teams = n, group = grid_blocks() / n;
+        const double delta = P.delta;
+        P.delta *= 8.0;
+        if (d_src_id) launch_grid<true>(P, teams, group, st);
+        else launch_grid<false>(P, teams, group, st);
+        P.delta = delta;
+        P.fallback = 1;
+    }
     if (c->cluster > 0) {
         const int cs = call_cluster(c, n);
         const int nc = std::min(nb, query_cluster_slots(cs));

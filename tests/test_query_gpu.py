@@ -113,3 +113,31 @@ def test_cluster_and_plain_forms_agree(graph):
     assert np.array_equal(out[QUERY_PLAIN][0], out[QUERY_CLUSTER][0])
     assert np.array_equal(out[QUERY_PLAIN][1][0], out[QUERY_CLUSTER][1][0])
     assert (out[QUERY_PLAIN][1][1] == out[QUERY_CLUSTER][1][1]).mean() > 0.999   # equal-distance ties
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 16, 17, 32, 33, 40])
+def test_whole_graph_searches_by_batch_size(n):
+    """MSAD batches of up to 32 run on an equal team of all the GPU's blocks per
+    query (odd shares, teams of 296 down to 9 blocks, frontiers that outgrow a
+    block's staging list), larger ones on clusters: the same distances as the
+    plain form, sources that explain them, and the next call unaffected."""
+    from svg_b200 import QUERY_CLUSTER, QUERY_PLAIN
+    pos, faces = meshgen.torus(1.0, 0.35, 400, 300, 0.02, seed=12)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    s.ConstructSVG(with_paths=False)
+    rng = np.random.default_rng(n)
+    sets = [rng.choice(m.vertNum, int(k), replace=False).astype(np.int32) for k in rng.integers(1, 60, n)]
+    weights = [rng.uniform(0, 0.2, len(x)) for x in sets]
+    first = s.msad_batch(sets, weights)
+    again = s.msad_batch(sets[::-1], weights[::-1])
+    s.set_query_form(QUERY_PLAIN)
+    plain = s.msad_batch(sets, weights)
+    s.set_query_form(QUERY_CLUSTER)
+    assert np.array_equal(first[0], plain[0])
+    assert np.array_equal(again[0][::-1], plain[0])
+    assert (first[1] == plain[1]).mean() > 0.999   # equal-distance ties
+    for q in range(n):
+        assert np.isin(first[1][q], sets[q]).all()
