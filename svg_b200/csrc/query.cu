@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include <cooperative_groups.h>
+#include <math_constants.h>
 
 #include "engine.h"
 
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kQThreads) k_query(QParams P) {
 constexpr int kCThreads = SVG_QC_THREADS;
 
 struct QCtl {
-    unsigned long long fmin[3];  // smallest waiting priority, by threshold move
+    unsigned long long fmin[3];  // smallest waiting priority, for the threshold move of that number
     int nearA[3];                // near list filled by the far split
     int farB[3];                 // far list filled by the split and the drain
     int nextX[3];                // next near list, by drain round
@@ -638,6 +639,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 ctl->touch = 1;
                 S.far[nf++] = s;
                 S.fflag[s] = fst;
+                ctl->fmin[0] = as_b(hdist(P.pos, s, tgt));
             } else {
                 // SVG.cu:358-364: assignments in listed order, the last weight of a repeated source wins
                 const int64_t b = P.set_off[q], e = P.set_off[q + 1];
@@ -654,6 +656,9 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                         S.far[nf++] = v;
                     }
                 }
+                unsigned long long m = kInfBits;
+                for (int i = 0; i < nf; ++i) m = min(m, S.ds[S.far[i]].d);
+                ctl->fmin[0] = m;
             }
             ctl->init_far = nf;
         }
@@ -665,6 +670,11 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
         bool over = false;
 
         // ---------------- main loop: move the threshold, drain near frontiers
+        // The smallest waiting priority is gathered on the way, from every
+        // vertex put or left in the far list (one whose priority fell below
+        // the threshold since makes it too small, which only costs an empty
+        // move): fmin[o] of this move was complete at the last barrier.
+        double thr = -CUDART_INF;
         for (;;) {
             // the far counter keeps counting past the list's capacity, so an
             // overflow shows in the value every block reads after the barrier
@@ -672,30 +682,27 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 over = true;
                 break;
             }
-            const int ob = o % 3;
-            unsigned long long m = kInfBits;
-            for (int i = gtid; i < farN; i += nthr) {
-                const int v = __ldcg(&far[i]);
-                const double d = kSSSD ? as_d(__ldcg(&S.dist[v])) : as_d(ld_ds(&S.ds[v]).d);
-                const double f = kSSSD ? d + hdist(P.pos, v, tgt) : d;
-                m = as_b(f) < m ? as_b(f) : m;
-            }
-            m = warp_min_u64(m);
-            if (lane == 0 && m != kInfBits) atomicMin(&ctl->fmin[ob], m);
+            if (farN == 0) break;
+            const int ob = o % 3, nb = (o + 1) % 3;
+            const double fmin = as_d(*(volatile unsigned long long*)&ctl->fmin[ob]);
+            if (kSSSD && as_d(__ldcg(&S.dist[tgt])) <= fmin) break;  // no waiting path can beat the target
+            const double settled = thr;
+            thr = fmin + P.delta;
             if (leader) {
-                const int nb = (o + 1) % 3;
-                ctl->fmin[nb] = kInfBits;
+                ctl->fmin[(o + 2) % 3] = kInfBits;
                 ctl->nearA[nb] = 0;
                 ctl->farB[nb] = 0;
             }
-            if (!team.sync()) return give_up(q);
-            if (farN == 0) break;
-            const double fmin = as_d(*(volatile unsigned long long*)&ctl->fmin[ob]);
-            if (kSSSD && as_d(__ldcg(&S.dist[tgt])) <= fmin) break;  // no waiting path can beat the target
-            const double thr = fmin + P.delta;
             stamp += 2;
             const uint32_t nst = stamp - 1, fst2 = stamp;
-            // split far: below the threshold -> near, the rest -> far2 (deduplicated)
+            unsigned long long waiting = kInfBits;
+            auto flush_waiting = [&]() {
+                const unsigned long long m = warp_min_u64(waiting);
+                if (lane == 0 && m != kInfBits) atomicMin(&ctl->fmin[nb], m);
+                waiting = kInfBits;
+            };
+            // split far: below the last threshold -> settled, below the new one
+            // -> near, the rest -> far2 (deduplicated)
             for (int base = gwarp * 32; base < farN; base += nthr) {
                 const int i = base + lane;
                 bool to_near = false, to_far = false;
@@ -704,12 +711,18 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                     v = __ldcg(&far[i]);
                     const double d = kSSSD ? as_d(__ldcg(&S.dist[v])) : as_d(ld_ds(&S.ds[v]).d);
                     const double f = kSSSD ? d + hdist(P.pos, v, tgt) : d;
-                    if (f < thr) to_near = atomicExch(&S.nflag[v], nst) != nst;
-                    else to_far = atomicExch(&S.fflag[v], fst2) != fst2;
+                    if (f < settled) {
+                    } else if (f < thr) {
+                        to_near = atomicExch(&S.nflag[v], nst) != nst;
+                    } else {
+                        to_far = atomicExch(&S.fflag[v], fst2) != fst2;
+                        waiting = min(waiting, as_b(f));
+                    }
                 }
                 put(s_near, to_near, v, &ctl->nearA[ob], near, P.nv);
                 put(s_far, to_far, v, &ctl->farB[ob], far2, P.list_cap);
             }
+            flush_waiting();
             if constexpr (kStaged) {
                 stage_flush(s_near, &ctl->nearA[ob], near, P.nv, &s_base);
                 stage_flush(s_far, &ctl->farB[ob], far2, P.list_cap, &s_base);
@@ -774,6 +787,8 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                             if (!__any_sync(0xffffffffu, maybe)) continue;
                             if (maybe) {
                                 bool improved = false;
+                                // (the positions arrive while the atomic is under way)
+                                const double f = kSSSD ? nd[j] + hdist(P.pos, w, tgt) : nd[j];
                                 if (kSSSD) {
                                     const unsigned long long old = atomicMin(&S.dist[w], as_b(nd[j]));
                                     improved = nd[j] < as_d(old);
@@ -795,9 +810,12 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                                     }
                                 }
                                 if (improved) {
-                                    const double f = kSSSD ? nd[j] + hdist(P.pos, w, tgt) : nd[j];
-                                    if (f < thr) to_next = atomicExch(&S.nflag[w], xst) != xst;
-                                    else to_far = atomicExch(&S.fflag[w], fst2) != fst2;
+                                    if (f < thr) {
+                                        to_next = atomicExch(&S.nflag[w], xst) != xst;
+                                    } else {
+                                        to_far = atomicExch(&S.fflag[w], fst2) != fst2;
+                                        waiting = min(waiting, as_b(f));
+                                    }
                                 }
                             }
                             if (kSSSD) {
@@ -809,6 +827,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                         }
                     }
                 }
+                flush_waiting();
                 if constexpr (kStaged) {
                     stage_flush(s_near, &ctl->nextX[gb], next, P.nv, &s_base);
                     stage_flush(s_far, &ctl->farB[ob], far, P.list_cap, &s_base);
@@ -863,9 +882,11 @@ __global__ void k_mean_weight(const double* w, int64_t n, double* out) {
     if (threadIdx.x == 0) atomicAdd(out, s[0]);
 }
 
-__global__ void k_fill(unsigned long long* p, size_t n, unsigned long long v) {
+// SSSD distances of every slot to +inf, one grid row per slot.
+__global__ void k_fill_slots(char* base, size_t slot_bytes, size_t n) {
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(base + blockIdx.y * slot_bytes);
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        p[i] = v;
+        p[i] = kInfBits;
 }
 
 size_t al256(size_t x) { return (x + 255) / 256 * 256; }
@@ -1044,13 +1065,24 @@ int query_cluster_slots(int csize) {
 }
 
 namespace {
+// Single-pair batches from this size on are served by 4-block clusters, twice
+// as many at once: such a search keeps few vertices in its frontier, so that
+// the lanes of 8 blocks are mostly idle, and touches too little of the graph to
+// thrash L2.  8 against 4 blocks: 2,048 pairs on the 750K torus 166 / 138 ms,
+// 1,000 on a 30K graph 9.1 / 6.1 ms, 500 on the 73K height field 9.5 / 7.3 ms;
+// but 100 pairs 14.4 / 22.7 ms on the 750K torus (fewer full rounds).
+constexpr int kSmallTeamQueries = 300;
+constexpr int kSmallTeam = 4;
+constexpr size_t kSmallTeamBytes = (size_t)4 << 30;  // most scratch of a context made for them
+
 // Cluster size of one call: a context made with `adaptive` serves a batch that
 // fits in the resident clusters of its size at that size (latency), and a
 // larger batch with 8-block clusters, which pack the SMs more fully
-// (throughput); otherwise the context's own size.
-int call_cluster(const svg_qctx* c, int n) {
+// (throughput), or 4-block ones (large single-pair batches, where the context
+// has slots for them); otherwise the context's own size.
+int call_cluster(const svg_qctx* c, int n, bool sssd) {
     if (!c->adaptive || c->cluster <= 8 || n <= query_cluster_slots(c->cluster)) return c->cluster;
-    return 8;
+    return sssd && n >= kSmallTeamQueries && c->slots > query_cluster_slots(8) ? kSmallTeam : 8;
 }
 }  // namespace
 
@@ -1065,6 +1097,14 @@ int query_slots_per_sm() {
     return per_sm;
 }
 
+namespace {
+int64_t list_capacity(int32_t nv) { return 2 * (int64_t)nv + 64; }
+size_t slot_size(int32_t nv) {
+    const size_t V = (size_t)nv;
+    return al256(8 * V) + al256(16 * V) + 4 * al256(4 * V) + 2 * al256(4 * (size_t)list_capacity(nv)) + al256(4 * V);
+}
+}  // namespace
+
 // Query scratch for `slots` concurrent queries of one graph: per slot the SSSD
 // distances (kept at +inf between queries), the MSAD {dist, src} pairs, the
 // stamp arrays and the frontier lists; one launch at a time may use it.
@@ -1075,8 +1115,8 @@ svg_qctx* qctx_create(svg_graph* g, int slots, cudaStream_t st, int cluster) {
     c->slots = std::max(1, slots);
     c->cluster = std::max(0, cluster);
     const size_t V = (size_t)g->nv;
-    c->list_cap = 2 * (int64_t)V + 64;
-    c->slot_bytes = al256(8 * V) + al256(16 * V) + 4 * al256(4 * V) + 2 * al256(4 * (size_t)c->list_cap) + al256(4 * V);
+    c->list_cap = list_capacity(g->nv);
+    c->slot_bytes = slot_size(g->nv);
     const size_t body = al256((size_t)c->slots * c->slot_bytes);
     const size_t ctl_at = body + al256(sizeof(uint32_t) * (size_t)c->slots) + 256;
     const size_t need = ctl_at + sizeof(QCtl) * (size_t)c->slots;
@@ -1091,9 +1131,8 @@ svg_qctx* qctx_create(svg_graph* g, int slots, cudaStream_t st, int cluster) {
     c->head = reinterpret_cast<int32_t*>(base + body + al256(sizeof(uint32_t) * (size_t)c->slots));
     c->ctl = base + ctl_at;
     SVG_CUDA(cudaMemsetAsync(base, 0, need, st));  // stamps and flags start at 0
-    for (int sl = 0; sl < c->slots; ++sl)          // SSSD distances start at +inf
-        k_fill<<<64, 256, 0, st>>>(reinterpret_cast<unsigned long long*>(base + (size_t)sl * c->slot_bytes), V,
-                                  kInfBits);
+    const dim3 grid((unsigned)std::min<size_t>((V + 255) / 256, 64), (unsigned)c->slots);
+    k_fill_slots<<<grid, 256, 0, st>>>(base, c->slot_bytes, V);  // SSSD distances start at +inf
     SVG_CUDA(cudaGetLastError());
     SVG_CUDA(cudaStreamSynchronize(st));
     return c;
@@ -1129,7 +1168,7 @@ void qctx_sssd(svg_qctx* c, int32_t n, const int32_t* d_s, const int32_t* d_t, d
     P.out = d_dist;
     SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t) * kHeadZeroed, st));
     if (c->cluster > 0) {
-        const int cs = call_cluster(c, n);
+        const int cs = call_cluster(c, n, true);
         launch_cluster<true, false>(P, std::min(std::min(n, c->slots), query_cluster_slots(cs)), cs, st);
     } else
         k_query<true, false><<<std::min(n, c->slots), kQThreads, 0, st>>>(P);
@@ -1164,7 +1203,7 @@ void qctx_msad(svg_qctx* c, int32_t n, const int64_t* d_off, const int32_t* d_sr
         P.fallback = 1;
     }
     if (c->cluster > 0) {
-        const int cs = call_cluster(c, n);
+        const int cs = call_cluster(c, n, false);
         const int nc = std::min(nb, query_cluster_slots(cs));
         if (d_src_id) launch_cluster<false, true>(P, nc, cs, st);
         else launch_cluster<false, false>(P, nc, cs, st);
@@ -1179,18 +1218,31 @@ void qctx_msad(svg_qctx* c, int32_t n, const int64_t* d_off, const int32_t* d_sr
 namespace {
 // The graph's own context for the synchronous batch entry points: as many
 // clusters as run at once (cluster form), or every resident block (plain form).
-svg_qctx* default_ctx(svg_graph* g) {
-    if (!g->qdefault) {
-        if (g->qform == SVG_QUERY_PLAIN) {
+// A large single-pair batch replaces a cluster context by one with slots for
+// 4-block clusters, within kSmallTeamBytes.
+svg_qctx* default_ctx(svg_graph* g, bool small_teams) {
+    if (g->qform == SVG_QUERY_PLAIN) {
+        if (!g->qdefault) {
             int dev = 0, sms = 0;
             SVG_CUDA(cudaGetDevice(&dev));
             SVG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             g->qdefault = qctx_create(g, query_slots_per_sm() * sms, lib_stream(), 0);
-        } else {
-            const int cs = query_cluster_size();
-            g->qdefault = qctx_create(g, std::max(query_cluster_slots(cs), query_cluster_slots(8)), lib_stream(), cs);
-            g->qdefault->adaptive = true;
         }
+        return g->qdefault;
+    }
+    const int cs = query_cluster_size();
+    int slots = std::max(query_cluster_slots(cs), query_cluster_slots(8));
+    if (small_teams)
+        slots = (int)std::max<size_t>((size_t)slots, std::min((size_t)query_cluster_slots(kSmallTeam),
+                                                              kSmallTeamBytes / std::max<size_t>(slot_size(g->nv), 1)));
+    if (g->qdefault && g->qdefault->slots < slots) {
+        SVG_CUDA(cudaStreamSynchronize(lib_stream()));
+        qctx_free(g->qdefault);
+        g->qdefault = nullptr;
+    }
+    if (!g->qdefault) {
+        g->qdefault = qctx_create(g, slots, lib_stream(), cs);
+        g->qdefault->adaptive = true;
     }
     return g->qdefault;
 }
@@ -1199,7 +1251,7 @@ svg_qctx* default_ctx(svg_graph* g) {
 
 svg_status run_sssd(svg_graph* g, int32_t n, const int32_t* d_s, const int32_t* d_t, double* d_dist) {
     if (n == 0) return SVG_OK;
-    qctx_sssd(default_ctx(g), n, d_s, d_t, d_dist, lib_stream());
+    qctx_sssd(default_ctx(g, n >= kSmallTeamQueries), n, d_s, d_t, d_dist, lib_stream());
     return SVG_OK;
 }
 
@@ -1207,7 +1259,7 @@ svg_status run_msad(svg_graph* g, int32_t n, const int64_t* d_off, const int32_t
                     double* d_dist, int32_t* d_src_id, int64_t total_srcs) {
     (void)total_srcs;
     if (n == 0) return SVG_OK;
-    qctx_msad(default_ctx(g), n, d_off, d_src, d_w, d_dist, d_src_id, lib_stream());
+    qctx_msad(default_ctx(g, false), n, d_off, d_src, d_w, d_dist, d_src_id, lib_stream());
     return SVG_OK;
 }
 

@@ -141,3 +141,23 @@ def test_whole_graph_searches_by_batch_size(n):
     assert (first[1] == plain[1]).mean() > 0.999   # equal-distance ties
     for q in range(n):
         assert np.isin(first[1][q], sets[q]).all()
+
+
+@pytest.mark.parametrize("n", [1, 14, 15, 34, 299, 300, 700])
+def test_single_pair_searches_by_batch_size(graph, n):
+    """Clusters of 16, 8 and 4 blocks by batch size (the last in a context with
+    more slots, made when first needed): the plain form's distances, also for
+    equal and unreachable pairs, and for a small batch after a large one."""
+    from svg_b200 import QUERY_CLUSTER, QUERY_PLAIN
+    s, m, cm, off, adj, dist = graph
+    rng = np.random.default_rng(n)
+    S = rng.integers(0, m.vertNum, n).astype(np.int32)
+    T = rng.integers(0, m.vertNum, n).astype(np.int32)
+    T[0] = S[0]
+    got = s.sssd_batch(S, T)
+    few = s.sssd_batch(S[:3], T[:3])
+    s.set_query_form(QUERY_PLAIN)
+    want = s.sssd_batch(S, T)
+    s.set_query_form(QUERY_CLUSTER)
+    assert np.array_equal(got, want)
+    assert np.array_equal(few, want[:3])
