@@ -1005,15 +1005,18 @@ void launch_cluster(const QParams& P, int nclusters, int csize, cudaStream_t st)
     SVG_CUDA(cudaLaunchKernelEx(&cfg, k_query_team<A, B, ClusterTeam>, P));
 }
 
-// Queries a grid-form launch serves at most, one team of blocks each.  Measured
-// (kernel time, clusters against teams): one MSAD on the 750K torus at K = 100
-// 8.85 / 1.38 ms, 4 of them 9.5 / 3.2, 16 19.6 / 11.3, 32 22.4 / 21.8; on the
-// 73K height field at K = 200 1 1.60 / 0.55 ms, 16 2.8 / 1.7, 32 3.1 / 3.2; on
-// a 30K graph 1 0.69 / 0.46 ms, 4 0.73 / 0.53, 16 1.05 / 0.81, 32 1.10 / 1.12.
-// A single-pair search touches too few vertices a round for that: a cluster
-// of 16 took 0.77 ms on the 750K torus, teams of 37 to 148 blocks 0.71-0.83,
-// and 0.18 against 0.24 ms on a 30K graph.
+// Queries a grid-form launch serves at most, one team of blocks each, and the
+// smallest graph it is used on.  Measured (whole calls, clusters against
+// teams): one MSAD on the 750K torus at K = 100 10.3 / 2.5 ms, 4 of them 12.8 /
+// 6.9; on the 73K height field at K = 200 1 1.60 / 0.52 ms, 4 1.97 / 1.21, 16
+// 4.0 / 3.1 (kernel time of 32 on the 750K torus 22.4 / 21.8 ms, on the 73K
+// height field 3.1 / 3.2); 10K vertices 1 0.27 / 0.20 ms, 16 0.63 / 0.55; 5K
+// vertices 1 0.170 / 0.173, 8 0.247 / 0.249; 1.5K vertices 1 0.106 / 0.119.
+// A single-pair search touches too few vertices a round for a wide team: a
+// cluster of 16 took 0.77 ms on the 750K torus, teams of 37 to 148 blocks
+// 0.71-0.83, and 0.18 against 0.24 ms on a 30K graph.
 constexpr int kGridQueries = 16;
+constexpr int kGridVertices = 6000;
 
 // Blocks of the grid form that run at once.
 int grid_blocks() {
@@ -1188,20 +1191,25 @@ void qctx_msad(svg_qctx* c, int32_t n, const int64_t* d_off, const int32_t* d_sr
     P.out_src = d_src_id;
     SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t) * kHeadZeroed, st));
     const int nb = std::min(n, c->slots);
-    if (c->adaptive && n <= std::min(kGridQueries, c->slots)) {
-        // Few queries: every block of the GPU serves them, an equal team each.
-        // The fewer the phases, the fewer the barriers: with teams this wide
-        // the extra relaxations of eight-fold buckets (1.27 V instead of 1.10 V
-        // on the 750K torus, in 66 phases instead of 179) cost less than they
-        // save (one MSAD 1.97 ms with two-fold buckets, 1.38 with eight-fold).
-        const int teams = n, group = grid_blocks() / n;
-        const double delta = P.delta;
-        P.delta *= 8.0;
+    // Bucket width: the fewer the phases, the fewer the barriers, against more
+    // vertices expanded more than once (8-fold buckets: 1.27 V instead of 1.10 V
+    // on the 750K torus, in 66 phases instead of 179).  A few searches on small
+    // graphs are all barriers: 4-fold buckets took 0.40 instead of 0.43 ms for
+    // a cluster on 20K vertices, 0.69 / 0.74 on 40K, but 1.67 / 1.60 on 73K.
+    const double delta = P.delta * (n <= kGridQueries && P.nv < 60000 ? 4.0 : 1.0);
+    if (c->adaptive && n <= std::min(kGridQueries, c->slots) && P.nv >= kGridVertices) {
+        // Few queries: every block of the GPU serves them, an equal team each,
+        // on small graphs of a block per 64 vertices (10K vertices 0.196 ms with
+        // 148 blocks, 0.209 with 296).  Wide teams want the widest buckets (one
+        // MSAD on the 750K torus: two-fold 1.97 ms of kernel time, eight-fold
+        // 1.38; 16-fold 5 % less again).
+        const int teams = n, group = std::min(grid_blocks() / n, P.nv / 64);
+        P.delta *= 16.0;
         if (d_src_id) launch_grid<true>(P, teams, group, st);
         else launch_grid<false>(P, teams, group, st);
-        P.delta = delta;
         P.fallback = 1;
     }
+    P.delta = delta;
     if (c->cluster > 0) {
         const int cs = call_cluster(c, n, false);
         const int nc = std::min(nb, query_cluster_slots(cs));

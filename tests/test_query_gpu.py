@@ -161,3 +161,25 @@ def test_single_pair_searches_by_batch_size(graph, n):
     s.set_query_form(QUERY_CLUSTER)
     assert np.array_equal(got, want)
     assert np.array_equal(few, want[:3])
+
+
+@pytest.mark.parametrize("nu,nv,n", [(100, 59, 2), (100, 60, 1), (101, 60, 16), (70, 43, 3)])
+def test_whole_graph_searches_around_the_smallest_team_graph(nu, nv, n):
+    """Graphs just below and above the size from which teams of all blocks
+    serve a small batch (clusters with wide buckets below it): the oracle's
+    distances."""
+    pos, faces = meshgen.torus(1.0, 0.35, nu, nv, 0.02, seed=3)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(30)
+    s.ConstructSVG(with_paths=False)
+    off, adj, dist = s.csr()
+    cm = CpuOracle().mesh(pos, faces)
+    rng = np.random.default_rng(n)
+    sets = [rng.choice(m.vertNum, 4, replace=False).astype(np.int32) for _ in range(n)]
+    weights = [rng.uniform(0, 0.2, 4) for _ in sets]
+    d, src = s.msad_batch(sets, weights)
+    for q in range(n):
+        rd, rs, _ = cm.msad(off, adj, dist, sets[q], weights[q])
+        assert np.all(np.abs(d[q] - rd) <= RTOL * np.maximum(rd, 1e-300))
