@@ -219,6 +219,32 @@ __global__ void k_dfma_rate(double* out, int iters, double b, double c) {
     if (s == 12345.678) out[0] = s;  // keeps the chains live; never true for these inputs
 }
 
+// Edges [first, first + n) of a graph as reference-layout nodes (svg_node, 40
+// bytes = five 8-byte words).  One thread per word: a warp writes 256
+// consecutive bytes, and the reads of the five threads of an edge are one
+// sector each.  Bound by the node bytes (12K height field at K = 200, 2.4 M
+// edges: the copy took 33 ms with the host assembling the nodes from three
+// arrays, of which this kernel replaces 20; it takes 0.05 ms itself).
+__global__ void __launch_bounds__(256) k_pack_nodes(const int32_t* __restrict__ adj, const double* __restrict__ dist,
+                                                    const PathEnd* __restrict__ paths, int64_t first, int64_t n,
+                                                    unsigned long long* __restrict__ out) {
+    const int64_t words = 5 * n;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = first + i / 5;
+        unsigned long long w;
+        switch ((int)(i % 5)) {
+            case 0: w = (unsigned long long)(uint32_t)adj[e]; break;  // adj, pad 0
+            case 1: w = (unsigned long long)__double_as_longlong(dist[e]); break;
+            case 2:
+                w = paths ? (unsigned long long)paths[e].src_edge | (unsigned long long)paths[e].dst_edge << 32 : ~0ull;
+                break;
+            case 3: w = paths ? (unsigned long long)__double_as_longlong(paths[e].src_x) : 0ull; break;
+            default: w = paths ? (unsigned long long)__double_as_longlong(paths[e].dst_x) : 0ull;
+        }
+        out[i] = w;
+    }
+}
+
 }  // namespace svgb
 
 using namespace svgb;
@@ -440,33 +466,28 @@ svg_status svg_graph_copy_csr(const svg_graph* g, int64_t* offsets, int32_t* adj
 svg_status svg_graph_copy_nodes(const svg_graph* g, int32_t* tails, svg_node* nodes) {
     return guarded([&]() -> svg_status {
         if (!g) throw SvgError{SVG_ERR_ARG, "null graph"};
-        std::vector<int64_t> off((size_t)g->nv + 1);
-        std::vector<int32_t> adj((size_t)g->nnz);
-        std::vector<double> dist((size_t)g->nnz);
-        std::vector<PathEnd> pe(g->with_paths ? (size_t)g->nnz : 0);
         cudaStream_t st = lib_stream();
-        SVG_CUDA(cudaMemcpyAsync(off.data(), g->off, sizeof(int64_t) * off.size(), cudaMemcpyDeviceToHost, st));
-        if (g->nnz) {
-            SVG_CUDA(cudaMemcpyAsync(adj.data(), g->adj, sizeof(int32_t) * adj.size(), cudaMemcpyDeviceToHost, st));
-            SVG_CUDA(cudaMemcpyAsync(dist.data(), g->dist, sizeof(double) * dist.size(), cudaMemcpyDeviceToHost, st));
-            if (g->with_paths)
-                SVG_CUDA(cudaMemcpyAsync(pe.data(), g->paths, sizeof(PathEnd) * pe.size(), cudaMemcpyDeviceToHost, st));
+        if (tails) {
+            std::vector<int64_t> off((size_t)g->nv + 1);
+            SVG_CUDA(cudaMemcpyAsync(off.data(), g->off, sizeof(int64_t) * off.size(), cudaMemcpyDeviceToHost, st));
+            SVG_CUDA(cudaStreamSynchronize(st));
+            for (int32_t v = 0; v < g->nv; ++v) tails[v] = (int32_t)(off[v + 1] - off[v]);
         }
-        SVG_CUDA(cudaStreamSynchronize(st));
-        for (int32_t v = 0; v < g->nv && tails; ++v) tails[v] = (int32_t)(off[v + 1] - off[v]);
-        for (int64_t i = 0; i < g->nnz && nodes; ++i) {
-            svg_node& n = nodes[i];
-            n.adj = adj[i];
-            n.pad_ = 0;
-            n.dist = dist[i];
-            if (g->with_paths) {
-                n.next_to_src_edge = pe[i].src_edge;
-                n.next_to_dst_edge = pe[i].dst_edge;
-                n.next_to_src_x = pe[i].src_x;
-                n.next_to_dst_x = pe[i].dst_x;
-            } else {
-                n.next_to_src_edge = n.next_to_dst_edge = 0xFFFFFFFFu;
-                n.next_to_src_x = n.next_to_dst_x = 0.0;
+        if (nodes && g->nnz) {
+            static_assert(sizeof(svg_node) == 40, "k_pack_nodes writes five words a node");
+            // assembled on the device, a bounded piece at a time
+            constexpr int64_t kPiece = (int64_t)8 << 20;  // nodes: 320 MB
+            const int64_t piece = std::min<int64_t>(g->nnz, kPiece);
+            DevBuf b;
+            b.reserve(sizeof(svg_node) * (size_t)piece);
+            for (int64_t first = 0; first < g->nnz; first += piece) {
+                const int64_t n = std::min(piece, g->nnz - first);
+                k_pack_nodes<<<(int)std::min<int64_t>((5 * n + 255) / 256, 4736), 256, 0, st>>>(
+                    g->adj, g->dist, g->with_paths ? static_cast<const PathEnd*>(g->paths) : nullptr, first, n,
+                    b.as<unsigned long long>());
+                SVG_CUDA(cudaGetLastError());
+                SVG_CUDA(cudaMemcpyAsync(nodes + first, b.p, sizeof(svg_node) * (size_t)n, cudaMemcpyDeviceToHost, st));
+                SVG_CUDA(cudaStreamSynchronize(st));
             }
         }
         return SVG_OK;
