@@ -77,7 +77,7 @@ struct PhaseOut {
     int32_t* st_windows;
     int32_t* st_maxq;
     int32_t* st_flags;
-    unsigned long long* acc;       // windows, generated, pseudo-sources, largest queues, largest source's windows
+    unsigned long long* acc;       // windows, generated, pseudo-sources, largest queues, largest source's windows, longest candidate list
     // Cooperative warps: warp 0 of each of the first coop_warps blocks takes
     // the heaviest sources order[0 .. coop_n) one at a time from its own
     // queue head (coop_work) and runs each with the whole warp, its two heaps
@@ -218,6 +218,7 @@ __device__ void finish_warp(LaneType& L, const PhaseOut& O, int v, unsigned amas
             O.cand_start[v] = (int64_t)base;
             O.cand_n[v] = n;
             O.deg[v] = min(n, L.C.K);
+            atomicMax(&O.acc[6], (unsigned long long)n);
             if (L.flags & kFlagUndefined) O.st_flags[v] |= 8;
         }
     }
@@ -488,12 +489,38 @@ __global__ void __launch_bounds__(256, SVG_TRACE_MIN_BLOCKS) k_trace(DevMesh M, 
     }
 }
 
-// Warp-per-source emission.
+// Bitonic sort of N (a power of two, at least 32) keys in shared memory by one
+// warp, each lane on whole pairs.
+template <class Key>
+__device__ __forceinline__ void warp_sort(Key* keys, int N, int lane) {
+    for (int k = 2; k <= N; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int p = lane; p < N / 2; p += 32) {
+                const int i = ((p & ~(j - 1)) << 1) | (p & (j - 1));
+                const Key a = keys[i], b = keys[i | j];
+                if ((a > b) == ((i & k) == 0)) {
+                    keys[i] = b;
+                    keys[i | j] = a;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// Warp-per-source emission: the candidates sorted by vertex id, the first K
+// written.  Bound by the sort's shared-memory passes, so what counts is warps
+// per SM and bytes per key: the launch holds room for the longest list there
+// is (not for the longest possible), and a list whose ids span less than 2^22
+// and which has at most 1,023 entries is sorted as 32-bit keys (id offset,
+// place).  73K height field K = 500 6.5 -> 1.1 ms, 750K torus K = 100
+// 4.0 -> 1.5 ms.
 __global__ void __launch_bounds__(256) k_emit(EmitParams P) {
     extern __shared__ unsigned long long sm_keys[];
     int lane = threadIdx.x & 31;
     int wib = threadIdx.x >> 5;
     unsigned long long* keys = sm_keys + (size_t)wib * P.smax;
+    uint32_t* short_keys = reinterpret_cast<uint32_t*>(keys);
     int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int nw = (gridDim.x * blockDim.x) >> 5;
     for (int r = gw; r < P.nsrc; r += nw) {
@@ -503,35 +530,33 @@ __global__ void __launch_bounds__(256) k_emit(EmitParams P) {
         int64_t start = P.cand_start[v];
         int N = 32;
         while (N < n) N <<= 1;
-        if (N > P.smax) {  // cannot happen: smax covers the largest vertex list
+        if (N > P.smax) {  // cannot happen: smax covers the longest list
             if (lane == 0) P.st_flags[v] |= 8;
             continue;
         }
-        for (int i = lane; i < N; i += 32)
-            keys[i] = i < n ? ((unsigned long long)(uint32_t)P.cand[start + i].u << 32) | (uint32_t)i
-                            : ~0ull;
-        __syncwarp();
-        for (int k = 2; k <= N; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < N; i += 32) {
-                    int ixj = i ^ j;
-                    if (ixj > i) {
-                        unsigned long long a = keys[i], b = keys[ixj];
-                        bool up = (i & k) == 0;
-                        if ((a > b) == up) {
-                            keys[i] = b;
-                            keys[ixj] = a;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
+        uint32_t lo = 0xFFFFFFFFu, hi = 0;
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t u = (uint32_t)P.cand[start + i].u;
+            lo = min(lo, u);
+            hi = max(hi, u);
         }
+        lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+        hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+        // (the padding key ~0 stays above every other: an offset of 2^22 - 1 would need place 1,023)
+        const bool small = n <= 1023 && hi - lo < 1u << 22;
+        for (int i = lane; i < N; i += 32) {
+            const uint32_t u = i < n ? (uint32_t)P.cand[start + i].u : 0u;
+            if (small) short_keys[i] = i < n ? (u - lo) << 10 | (uint32_t)i : ~0u;
+            else keys[i] = i < n ? (unsigned long long)u << 32 | (uint32_t)i : ~0ull;
+        }
+        __syncwarp();
+        if (small) warp_sort(short_keys, N, lane);
+        else warp_sort(keys, N, lane);
         int deg = min(n, P.K);
         int64_t base = P.off[v];
         int fl = 0;
         for (int i = lane; i < deg; i += 32) {
-            int idx = (int)(keys[i] & 0xFFFFFFFFu);
+            const int idx = small ? (int)(short_keys[i] & 1023u) : (int)(keys[i] & 0xFFFFFFFFu);
             Cand c = P.cand[start + idx];
             P.adj[base + i] = c.u;
             P.dist[base + i] = c.dist;
@@ -1404,7 +1429,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     DevBuf b_padj, b_pdist, b_ppath, b_tails;
     int32_t retry_n = 0;
     int32_t retry_host_cap_log2_v = lay.vcap_log2 + 1, retry_host_cap_log2_s = lay.scap_log2 + 2;
-    int32_t smax_vlimit = lay.vlimit;
+    unsigned long long longest = 0;  // candidate list
     int64_t scratch_bytes = (int64_t)(lane_bytes(lay) * lay.lanes);
 
     if (plain) {
@@ -1449,8 +1474,14 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
             SVG_CUDA(cudaGetLastError());
             SVG_CUDA(cudaMemcpyAsync(&retry_n, d_retry_n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
             unsigned long long used = 0;
-            SVG_CUDA(cudaMemcpyAsync(&used, d_cand_used, sizeof(used), cudaMemcpyDeviceToHost, st));
-            SVG_CUDA(cudaStreamSynchronize(st));
+            auto read_lists = [&]() {  // candidate pool use, longest list
+                unsigned long long w[3];
+                SVG_CUDA(cudaMemcpyAsync(w, d_acc + 6, sizeof(w), cudaMemcpyDeviceToHost, st));
+                SVG_CUDA(cudaStreamSynchronize(st));
+                longest = w[0];
+                used = w[2];
+            };
+            read_lists();
             if (retry_n > 0) {
                 // Sources whose tables filled: rerun them with 2x vertex and 4x split tables.
                 LaneConfig C2 = C;
@@ -1495,11 +1526,9 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                 SVG_CUDA(cudaGetLastError());
                 int32_t again = 0;
                 SVG_CUDA(cudaMemcpyAsync(&again, d_work + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-                SVG_CUDA(cudaMemcpyAsync(&used, d_cand_used, sizeof(used), cudaMemcpyDeviceToHost, st));
-                SVG_CUDA(cudaStreamSynchronize(st));
+                read_lists();
                 if (again > 0)
                     throw SvgError{SVG_ERR_NOMEM, "a source outgrew the enlarged retry tables"};
-                smax_vlimit = std::max(smax_vlimit, l2.vlimit);
             }
             if ((int64_t)used <= cap) break;
             if (attempt >= 2) throw SvgError{SVG_ERR_NOMEM, "candidate pool kept overflowing"};
@@ -1549,7 +1578,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         E.path = reinterpret_cast<PathEnd*>(g->paths);
         E.st_flags = g->st_flags;
         int smax = 32;
-        while (smax < smax_vlimit) smax <<= 1;
+        while (smax < (int64_t)longest) smax <<= 1;
         E.smax = smax;
         int wpb = (int)std::max<int64_t>(1, std::min<int64_t>(8, (96 * 1024) / ((int64_t)smax * 8)));
         size_t smem = (size_t)wpb * smax * 8;
@@ -1609,7 +1638,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         P.wpb = cap_wpb;
         P.emit_smem = cap_emit_smem;
         P.smax = 32;
-        while (P.smax < smax_vlimit) P.smax <<= 1;
+        while (P.smax < (int64_t)longest) P.smax <<= 1;
         P.with_paths = g->with_paths;
         P.lay = lay;
         P.scratch_bytes = scratch_bytes;

@@ -162,6 +162,12 @@ __device__ __forceinline__ double hyp(double x, double y) { return sqrt(x * x + 
 __device__ __forceinline__ bool to_left(double px, double py, double p0x, double p0y, double p1x, double p1y) {
     double ax = p1x - p0x, ay = p1y - p0y;
     double bx = px - p0x, by = py - p0y;
+    // The normalised vectors' product has the sign of the plain one wherever
+    // that exceeds its terms' rounding: normalising changes each term by less
+    // than 2^-50 of itself.  Only the rest (and NaN, infinities, underflow to
+    // zero) takes the reference's two square roots and four divisions.
+    const double u = ax * by, w = ay * bx, c = u - w;
+    if (fabs(c) > 0x1p-45 * (fabs(u) + fabs(w))) return c > 0.0;
     double la = sqrt(ax * ax + ay * ay);
     if (!(fabs(la) < 1e-12)) { ax /= la; ay /= la; }
     double lb = sqrt(bx * bx + by * by);
