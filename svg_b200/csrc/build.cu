@@ -1306,9 +1306,14 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     // set the tail); the rest keep vertex order, so that the sources in
     // flight together stay neighbours on the mesh and share its lines in L2
     // (full heaviest-first order is 3 % slower on the 750K torus, vertex
-    // order 13 % slower on the 72.9K height field).
+    // order 13 % slower on the 72.9K height field).  Sources of about the same
+    // cost in more than 3.5 waves keep vertex order altogether: 200K torus
+    // K = 100 67.6 / 67.0 ms, 750K torus 235.5 / 230.9 ms; but 120K torus
+    // K = 200 (2.9 waves) 119.0 / 121.3 ms, and the 200K height field, uneven,
+    // 69.6 / 71.6 ms.
     const int64_t head = std::min<int64_t>(nsrc, (int64_t)lay.lanes * o.heavy_waves);
-    const bool by_cost = !plain && o.heavy_first && m->cost_K == K && nsrc > 0;
+    const bool many_even = m->cost_even && 2 * (int64_t)nsrc > 7 * (int64_t)lay.lanes;
+    const bool by_cost = !plain && o.heavy_first && m->cost_K == K && nsrc > 0 && !(many_even && o.coop_sources == 0);
     DevBuf b_plan;
     if (by_cost && o.coop_sources == 0 && !one_wave) {
         CostOrder P{};
