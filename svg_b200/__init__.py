@@ -332,9 +332,9 @@ class SVG:
             _check(lib().svg_graph_copy_csr(self._g, off.ctypes.data_as(_P), adj.ctypes.data_as(_P),
                                             dist.ctypes.data_as(_P)))
             return off[:nv + 1], adj[:nnz], dist[:nnz]
-        off = np.zeros(nv + 1, np.int64)
-        adj = np.zeros(max(nnz, 1), np.int32)
-        dist = np.zeros(max(nnz, 1))
+        off = np.empty(nv + 1, np.int64)
+        adj = np.empty(max(nnz, 1), np.int32)
+        dist = np.empty(max(nnz, 1))
         _check(lib().svg_graph_copy_csr(self._g, off.ctypes.data_as(_P), adj.ctypes.data_as(_P),
                                         dist.ctypes.data_as(_P)))
         return off, adj[:nnz], dist[:nnz]
@@ -342,8 +342,8 @@ class SVG:
     def CopySVGToHost(self):
         """(offsets, nodes): reference-layout rows packed in CSR order."""
         nv, nnz, _ = self.counts()
-        tails = np.zeros(nv, np.int32)
-        nodes = np.zeros(max(nnz, 1), NODE_DTYPE)
+        tails = np.empty(nv, np.int32)
+        nodes = np.empty(max(nnz, 1), NODE_DTYPE)
         _check(lib().svg_graph_copy_nodes(self._g, tails.ctypes.data_as(_P), nodes.ctypes.data_as(_P)))
         off = np.zeros(nv + 1, np.int64)
         np.cumsum(tails, out=off[1:])
@@ -366,7 +366,7 @@ class SVG:
     def sssd_batch(self, s, t) -> np.ndarray:
         s = np.ascontiguousarray(s, np.int32)
         t = np.ascontiguousarray(t, np.int32)
-        d = np.zeros(len(s))
+        d = np.empty(len(s))
         _check(lib().svg_sssd_batch(self._g, len(s), s, t, d))
         return d
 
@@ -384,8 +384,10 @@ class SVG:
             w = np.zeros(len(srcs))
         else:
             w = np.ascontiguousarray(np.concatenate(weights) if n else np.zeros(0), np.float64)
-        dist = np.zeros(n * V)
-        sid = np.zeros(n * V, np.int32) if with_src else None
+        # (the library writes every element: clearing the arrays first took as
+        # long as copying the results into them)
+        dist = np.empty(n * V)
+        sid = np.empty(n * V, np.int32) if with_src else None
         _check(lib().svg_msad_batch(self._g, n, off, srcs.ctypes.data_as(_P), w.ctypes.data_as(_P), dist,
                                     sid.ctypes.data_as(_P) if with_src else None))
         dist = dist.reshape(n, V)
@@ -400,9 +402,9 @@ class SVG:
         srcs = np.ascontiguousarray(np.concatenate(sets) if n else np.zeros(0), np.int32)
         w = np.zeros(len(srcs)) if weights is None else \
             np.ascontiguousarray(np.concatenate(weights) if n else np.zeros(0), np.float64)
-        dist = np.zeros(n * V)
-        sid = np.zeros(n * V, np.int32)
-        par = np.zeros(n * V, np.int32)
+        dist = np.empty(n * V)
+        sid = np.empty(n * V, np.int32)
+        par = np.empty(n * V, np.int32)
         _check(lib().svg_msad_batch_paths(self._g, n, off, srcs.ctypes.data_as(_P), w.ctypes.data_as(_P), dist,
                                           sid.ctypes.data_as(_P), par.ctypes.data_as(_P)))
         return dist.reshape(n, V), sid.reshape(n, V), par.reshape(n, V)
