@@ -108,14 +108,15 @@ typedef struct svg_build_opts {
                                  share), 0 none (the default) */
     int32_t coop_warps;       /* warps that run them (0 automatic) */
     int32_t vote_wait;        /* batched: most loop iterations a lane waits for the warp's vote to pick its
-                                 kind of step (0 = 8) */
+                                 kind of step (0 = 16) */
     int32_t heavy_waves;      /* batched: waves of lanes filled heaviest-first before vertex order (0 = 2) */
     int32_t heap_factor;      /* batched: first-pass physical window heap = heap_factor x K entries (0 = 3);
                                  a source that outgrows it is re-run with the full 1023 */
     int32_t autotune;         /* batched: 1 = use the parameters svg_build_autotune cached on this mesh for
                                  this K (if any) in place of the fields above and of blocks */
-    int32_t coop_tail;        /* batched: 1 (default) = once the work queue is drained, a warp left with one
-                                 running lane finishes that lane's source on all 32 threads; 0 = off */
+    int32_t coop_tail;        /* accepted and without effect: a drained queue's last lane of a warp once went
+                                 on as a cooperative warp, whose steps now take longer (4.6 us) than a lone
+                                 lane's (4.0 us) */
     int32_t graph;            /* batched: 1 = the build's device work (memsets, window propagation, offsets
                                  scan, emission, copies into the graph's buffers) is captured in a CUDA graph
                                  kept with the mesh, and later builds of the mesh with the same options

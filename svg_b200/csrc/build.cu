@@ -86,9 +86,6 @@ struct PhaseOut {
     int32_t coop_n;
     int32_t coop_warps;
     int32_t* coop_work;
-    // 1: once the work queue is drained, a warp left with one running lane
-    // finishes that lane's source in the cooperative form
-    int32_t coop_tail;
     // lanes of each warp that run sources (the lane scratch is laid out for
     // them alone: lane l of warp w has the scratch of index w * warp_lanes + l)
     int32_t warp_lanes;
@@ -266,7 +263,6 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
     int v = r < O.nsrc ? O.order[r] : -1;
     if (v >= 0) L.begin(v, false);
     int waited = 0;
-    int adopt = -1;
     for (;;) {
         const int act = v >= 0 ? L.template take<SVG_ICH_INLINE_STALE>() : -1;
         const unsigned m0 = __ballot_sync(kFull, act == Lane::kActWindow);
@@ -280,14 +276,6 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
         } else {
             const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
             chosen = (c0 >= c1 && c0 >= c2) ? Lane::kActWindow : (c1 >= c2 ? Lane::kActPseudo : Lane::kActDone);
-        }
-        if (O.coop_tail && O.warp_lanes > 1 && m2 == 0 && __popc(m0 | m1) == 1 &&
-            __ballot_sync(kFull, v < 0) == ~(m0 | m1)) {
-            // The queue is drained (every other lane that runs sources found it
-            // empty) and one lane still runs a source: the whole warp adopts it
-            // below.
-            adopt = __ffs(m0 | m1) - 1;
-            break;
         }
         const unsigned amask = chosen == Lane::kActWindow ? m0 : (chosen == Lane::kActPseudo ? m1 : m2);
         if (chosen == Lane::kActDone) finish_warp(L, O, v, amask);  // the whole warp exports
@@ -304,14 +292,11 @@ __global__ void SVG_ICH_BOUNDS k_ich_batched(LaneConfig C, PhaseOut O) {
             ++waited;
         }
     }
-    if (runs) L.save_epoch(lid);  // adoption below keeps lane `adopt`'s epoch: no begin() runs there
-    if (adopt >= 0) {
-        CoopLane W(C, wbase);
-        W.adopt(L, adopt);
-        while (!W.step()) {
-        }
-        finish_warp(W, O, __shfl_sync(kFull, v, adopt), 1u << adopt);  // lane `adopt`'s scratch; it owns it
-    }
+    // A warp left with one running lane goes on as it is: a lone lane's step
+    // takes 4.0 us, the cooperative form's 4.6.  Handing that lane's source to
+    // the whole warp cost 2.62 against 2.51 ms at 5K vertices K=50, 43.8
+    // against 38.0 at 12K K=200, 14.1 against 13.7 at 30K K=100.
+    if (runs) L.save_epoch(lid);
 }
 
 // BuildGeodesicPathTo(vertex) (ICHDevice.cu:336-480), the full back-trace the
@@ -873,7 +858,13 @@ svg_build_opts effective_options(const svg_mesh* m, const svg_build_opts& o) {
                 e.coop_tail = t.opts.coop_tail;
             }
     }
-    if (e.vote_wait <= 0) e.vote_wait = 8;
+    // A lane's step is dearer the more lanes of its warp take it, and a step
+    // of one or two waiting lanes costs the others a whole step's latency: the
+    // rarer kinds are let gather for up to 16 steps.  Build kernel, ms, at 4 /
+    // 8 / 16 / 32: 5K vertices K=50 2.50 / 2.51 / 2.55 / 2.58, 30K K=100 14.1
+    // / 13.7 / 13.6 / 13.5, 72.9K K=500 425 / 409 / 401 / 404, 750K K=100 237 /
+    // 229 / 227 / 227.
+    if (e.vote_wait <= 0) e.vote_wait = 16;
     if (e.heavy_waves <= 0) e.heavy_waves = 2;
     if (e.heap_factor <= 0) e.heap_factor = 3;
     return e;
@@ -1357,7 +1348,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         // fewer and shorter memory round trips per window.
         // The automatic share needs the costs of a build at this K: a K/10 probe
         // ranks the heaviest sources poorly (on the 72.9K height field its top
-        // 200 hold 27 of K=500's top 200), and the tail adoption covers them.
+        // 200 hold 27 of K=500's top 200).
         if (o.coop_sources > 0 || (o.coop_sources < 0 && !m->cost_probe)) {
             double total = 0.0;
             for (int32_t i = 0; i < nsrc; ++i) total += (double)cost[(size_t)(sb + i)];
@@ -1423,7 +1414,6 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     O.coop_n = coop_n;
     O.coop_warps = coop_warps;
     O.coop_work = d_work + 4;
-    O.coop_tail = o.coop_tail != 0 ? 1 : 0;
     O.warp_lanes = warp_lanes;
 
     cudaEvent_t ev[4];
@@ -1711,7 +1701,7 @@ svg_status run_autotune(svg_mesh* m, const svg_build_opts& in, int32_t max_trial
     base.coop_sources = 0;
     base.coop_warps = 0;
     base.coop_tail = 1;
-    base.vote_wait = 8;
+    base.vote_wait = 16;
     base.heavy_waves = 2;
     base.heap_factor = 3;
     base.blocks = 0;
@@ -1785,7 +1775,7 @@ svg_status run_autotune(svg_mesh* m, const svg_build_opts& in, int32_t max_trial
             consider(o);
         }
     }
-    for (int32_t w : {4, 16}) {
+    for (int32_t w : {8, 32}) {
         svg_build_opts o = best;
         o.vote_wait = w;
         consider(o);
@@ -1798,11 +1788,6 @@ svg_status run_autotune(svg_mesh* m, const svg_build_opts& in, int32_t max_trial
     for (int32_t f : {2, 4}) {
         svg_build_opts o = best;
         o.heap_factor = f;
-        consider(o);
-    }
-    {  // the drained-queue adoption off
-        svg_build_opts o = best;
-        o.coop_tail = 0;
         consider(o);
     }
     bool found = false;

@@ -348,18 +348,15 @@ struct LaneT {
         vtab_ = C.vtab + ((size_t)l << C.vcap_log2);
         stab_ = C.stab + ((size_t)l << C.scap_log2);
     }
-    // The cooperative form keeps its source's two heaps in shared memory
-    // (sheap: wstride window entries, then pstride pseudo-source entries), or,
-    // for a source it adopted from a lane (sheap null), in that lane's scratch.
+    // The cooperative form keeps its source's two heaps in shared memory:
+    // wstride window entries, then pstride pseudo-source entries.
     HeapEntry* sheap = nullptr;
     __device__ __forceinline__ HeapEntry* WH() const {
-        if constexpr (kCoop)
-            if (sheap) return sheap;
+        if constexpr (kCoop) return sheap;
         return wheap_;
     }
     __device__ __forceinline__ HeapEntry* PH() const {
-        if constexpr (kCoop)
-            if (sheap) return sheap + C.wstride;
+        if constexpr (kCoop) return sheap + C.wstride;
         return pheap_;
     }
     __device__ __forceinline__ WinPay* WP() const { return wpool_; }
@@ -399,56 +396,6 @@ struct LaneT {
     __device__ LaneT(const LaneConfig& c, int gtid) : C(c) {
         set_scratch(gtid);
         epoch = C.epochs[gtid];
-    }
-
-    // Cooperative form: take over the source lane o of this warp is running
-    // in the one-thread form (every thread calls it; the state comes from
-    // lane o by shuffles, the scratch and heaps stay lane o's, and the action
-    // lane o has pending becomes the warp's).
-    template <class Other>
-    __device__ void adopt(const Other& L, int o) {
-        constexpr unsigned kFull = 0xFFFFFFFFu;
-        sheap = nullptr;
-        set_scratch(__shfl_sync(kFull, L.lid, o));
-        wsize = __shfl_sync(kFull, L.wsize, o);
-        psize = __shfl_sync(kFull, L.psize, o);
-        nfree = __shfl_sync(kFull, L.nfree, o);
-        nfresh = __shfl_sync(kFull, L.nfresh, o);
-        ftop = __shfl_sync(kFull, L.ftop, o);
-        vcount = __shfl_sync(kFull, L.vcount, o);
-        scount = __shfl_sync(kFull, L.scount, o);
-        epoch = __shfl_sync(kFull, L.epoch, o);
-        source = __shfl_sync(kFull, L.source, o);
-        src_birth = __shfl_sync(kFull, L.src_birth, o);
-        total = __shfl_sync(kFull, L.total, o);
-        flags = __shfl_sync(kFull, L.flags, o);
-        done = __shfl_sync(kFull, (int)L.done, o) != 0;
-        pk_valid = __shfl_sync(kFull, (int)L.pk_valid, o) != 0;
-        pk_proc = __shfl_sync(kFull, (int)L.pk_proc, o) != 0;
-        pk_init = __shfl_sync(kFull, (int)L.pk_init, o) != 0;
-        pk_act = __shfl_sync(kFull, L.pk_act, o);
-        // the slots of lane o, read by every thread before any writes its own
-        copy_async_wait();
-        __syncwarp();
-        const int t = (threadIdx.x & ~31) + o;
-        const LaneSmem& G = g_lane_smem;
-        const int sw = G.windows[t], sp = G.pseudos[t], sg = G.generated[t], smw = G.maxw[t], smp = G.maxp[t];
-        const long long sst = G.steps[t];
-        const double k = G.pkey[t];
-        const int32_t id = G.pid[t];
-        const uint32_t bits = G.pbits[t];
-        const int4 p0 = G.pay[0][t], p1 = G.pay[1][t], p2 = G.pay[2][t];
-        __syncwarp();
-        st_windows() = sw;
-        st_pseudos() = sp;
-        st_generated() = sg;
-        st_maxw() = smw;
-        st_maxp() = smp;
-        st_steps() = sst;
-        set_pending(k, id, bits);
-        g_lane_smem.pay[0][threadIdx.x] = p0;
-        g_lane_smem.pay[1][threadIdx.x] = p1;
-        g_lane_smem.pay[2][threadIdx.x] = p2;
     }
 
     // ---------------------------------------------------------- tables
