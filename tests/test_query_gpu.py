@@ -117,7 +117,7 @@ def test_cluster_and_plain_forms_agree(graph):
 
 @pytest.mark.parametrize("n", [1, 2, 3, 16, 17, 32, 33, 40])
 def test_whole_graph_searches_by_batch_size(n):
-    """MSAD batches of up to 32 run on an equal team of all the GPU's blocks per
+    """MSAD batches of up to 16 run on an equal team of all the GPU's blocks per
     query (odd shares, teams of 296 down to 9 blocks, frontiers that outgrow a
     block's staging list), larger ones on clusters: the same distances as the
     plain form, sources that explain them, and the next call unaffected."""
@@ -183,3 +183,32 @@ def test_whole_graph_searches_around_the_smallest_team_graph(nu, nv, n):
     for q in range(n):
         rd, rs, _ = cm.msad(off, adj, dist, sets[q], weights[q])
         assert np.all(np.abs(d[q] - rd) <= RTOL * np.maximum(rd, 1e-300))
+
+
+@pytest.mark.parametrize("count", [31, 32, 33, 64, 1000])
+@pytest.mark.parametrize("n", [1, 20])
+def test_source_lists_with_repeats(n, count):
+    """Source lists around one, two and many rounds of 32 entries, their sources
+    listed several times within a round and across rounds, by teams of all blocks
+    (n = 1) and clusters: the last weight counts, as in the plain form."""
+    from svg_b200 import QUERY_CLUSTER, QUERY_PLAIN
+    pos, faces = meshgen.torus(1.0, 0.35, 100, 70, 0.02, seed=14)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    s.ConstructSVG(with_paths=False)
+    rng = np.random.default_rng(count)
+    pool = rng.choice(m.vertNum, max(2, count // 3), replace=False)
+    sets = [rng.choice(pool, count).astype(np.int32) for _ in range(n)]
+    weights = [rng.uniform(0, 0.3, count) for _ in sets]
+    d, src = s.msad_batch(sets, weights)
+    s.set_query_form(QUERY_PLAIN)
+    pd, ps = s.msad_batch(sets, weights)
+    s.set_query_form(QUERY_CLUSTER)
+    assert np.array_equal(d, pd)
+    assert (src == ps).mean() > 0.999   # equal-distance ties
+    for q in range(n):
+        last = dict(zip(sets[q].tolist(), weights[q].tolist()))
+        for v, w in last.items():
+            assert d[q][v] <= w and (src[q][v] == v) == (d[q][v] == w)
