@@ -336,3 +336,19 @@ def test_work_order_does_not_change_the_graph():
             assert np.array_equal(x, y)
     mem = svg_b200.device_memory()
     assert mem["in_use"] > 0 and mem["peak"] >= mem["in_use"]
+
+
+@pytest.mark.parametrize("K", [300, 1000, 1500])
+def test_emission_of_short_and_long_candidate_lists(K):
+    """Lists of up to 1,023 candidates are sorted as 32-bit keys, longer ones as
+    64-bit keys (a dome: no saddle vertex, so every vertex reached is a
+    candidate; sources near its middle): the plain form's rows."""
+    k = 56
+    rng = np.random.default_rng(3)
+    y, x = np.mgrid[0:k, 0:k] + rng.uniform(-0.2, 0.2, (2, k, k))
+    pos = np.stack([x, y, -0.004 * ((x - 28) ** 2 + (y - 28) ** 2)], -1).reshape(-1, 3)
+    i = (np.arange(k - 1)[:, None] * k + np.arange(k - 1)).ravel()
+    faces = np.concatenate([np.stack([i, i + 1, i + k], 1), np.stack([i + 1, i + k + 1, i + k], 1)]).astype(np.int32)
+    out = [gpu_build(pos, faces, K, mode, source_begin=1500, source_end=1540)[:2] for mode in (MODE_BATCHED, MODE_PLAIN)]
+    assert np.diff(out[0][0]).max() == K
+    assert compare_rows(*out[0], *out[1]) == []
