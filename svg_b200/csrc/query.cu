@@ -1091,6 +1091,12 @@ namespace {
 constexpr int kSmallTeamQueries = 300;
 constexpr int kSmallTeam = 4;
 constexpr size_t kSmallTeamBytes = (size_t)4 << 30;  // most scratch of a context made for them
+// Such batches keep the GPU busy whatever the phases, so on graphs of this size
+// and up narrower buckets pay: fewer vertices are expanded more than once.
+// Buckets of one mean edge against half of it, 2,000 pairs: 5K vertices 2.88 /
+// 2.95 ms, 30K 10.8 / 10.8 (300: 2.45 / 2.37), 73K 26.6 / 25.2, 750K 134 / 126;
+// a quarter 25.8 on 73K and 125 on 750K.  A single pair 0.28 / 0.31 on 30K.
+constexpr int kNarrowVertices = 30000;
 
 // Cluster size of one call: a context made with `adaptive` serves a batch that
 // fits in the resident clusters of its size at that size (latency), and a
@@ -1186,6 +1192,7 @@ void qctx_sssd(svg_qctx* c, int32_t n, const int32_t* d_s, const int32_t* d_t, d
     SVG_CUDA(cudaMemsetAsync(P.head, 0, sizeof(int32_t) * kHeadZeroed, st));
     if (c->cluster > 0) {
         const int cs = call_cluster(c, n, true);
+        if (cs == kSmallTeam && n >= kSmallTeamQueries && P.nv >= kNarrowVertices) P.delta *= 0.5;
         launch_cluster<true, false>(P, std::min(std::min(n, c->slots), query_cluster_slots(cs)), cs, st);
     } else
         k_query<true, false><<<std::min(n, c->slots), kQThreads, 0, st>>>(P);

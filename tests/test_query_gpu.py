@@ -212,3 +212,22 @@ def test_source_lists_with_repeats(n, count):
         last = dict(zip(sets[q].tolist(), weights[q].tolist()))
         for v, w in last.items():
             assert d[q][v] <= w and (src[q][v] == v) == (d[q][v] == w)
+
+
+@pytest.mark.parametrize("nu,nv", [(149, 201), (150, 200)])
+def test_large_pair_batches_around_the_narrow_bucket_size(nu, nv):
+    """300 pairs on graphs just below and at the size from which such batches
+    use narrower buckets: the plain form's distances."""
+    from svg_b200 import QUERY_CLUSTER, QUERY_PLAIN
+    pos, faces = meshgen.torus(1.0, 0.35, nu, nv, 0.02, seed=15)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    s.ConstructSVG(with_paths=False)
+    rng = np.random.default_rng(nv)
+    S, T = rng.integers(0, m.vertNum, (2, 300)).astype(np.int32)
+    got = s.sssd_batch(S, T)
+    s.set_query_form(QUERY_PLAIN)
+    assert np.array_equal(got, s.sssd_batch(S, T))
+    s.set_query_form(QUERY_CLUSTER)
