@@ -859,7 +859,7 @@ def run_queries(args):
             "forms": out,
             "msad_batch_speedup_cluster_vs_plain": out["cluster"]["msad_batch_qps"] / out["plain"]["msad_batch_qps"],
             "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
-                         "frac": round(ach / peak, 4), "traffic": None, "kernel": "k_query_cluster (MSAD)",
+                         "frac": round(ach / peak, 4), "traffic": None, "kernel": "k_query_team (MSAD)",
                          "algorithmic_bytes_per_query": bytes_q,
                          "peak_source": "measured" if peaks.get("hbm_gbs") else "fallback"},
             "clocks": ck}

@@ -179,8 +179,9 @@ svg_status svg_graph_source_stats(const svg_graph* g, int32_t* windows, int32_t*
 void svg_graph_free(svg_graph* g);
 
 /* Kernel form of the query calls on this graph.  CLUSTER (default): one query
- * per thread-block cluster of 8-16 SMs, few queries in flight so that their
- * state stays in L2.  PLAIN: one query per thread block, the reference's
+ * per thread-block cluster of 4-16 blocks, few queries in flight so that their
+ * state stays in L2; up to 16 whole-graph searches on a graph of 6,000 vertices
+ * and more share all blocks of the GPU.  PLAIN: one query per thread block, the reference's
  * one-search-at-a-time form (SVG::SolveSSSD / SolveMSAD, SVG.cu:241-413),
  * kept as the baseline.  Results are the same in both forms. */
 enum { SVG_QUERY_CLUSTER = 0, SVG_QUERY_PLAIN = 1 };
