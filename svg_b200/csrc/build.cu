@@ -1303,7 +1303,8 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
     DevBuf b_order, b_misc, b_cand, b_candstart;
     int32_t coop_n = 0, coop_warps = 0;
     // what a capture of this build as a graph needs (see BuildGraph)
-    size_t cap_coop_smem = 0, cap_emit_smem = 0;
+    size_t coop_smem = 0, coop_room = 0;  // the cooperative warps' heaps, and the shared memory there is for them
+    size_t cap_emit_smem = 0;
     int cap_eb = 0, cap_wpb = 0, cap_attempts = 0;
     int64_t cap_pool = 0;
     b_order.reserve(sizeof(int32_t) * (size_t)std::max(nsrc, 1));
@@ -1385,6 +1386,19 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                 {o.coop_warps > 0 ? (int64_t)o.coop_warps : std::max<int64_t>(1, n / 2), n, warps / 2,
                  (int64_t)blocks});
             if (coop_warps <= 0) coop_n = 0;
+            // Their heaps (window then pseudo-source entries) lie in shared
+            // memory beside the lanes' state: heaps that a block could hold by
+            // themselves but not with it leave their sources to the lanes.
+            if (coop_n > 0) {
+                coop_smem = ((size_t)C.wstride + (size_t)C.pstride) * sizeof(HeapEntry);
+                cudaFuncAttributes fa{};
+                SVG_CUDA(cudaFuncGetAttributes(&fa, k_ich_batched));
+                coop_room = prop.sharedMemPerBlockOptin - fa.sharedSizeBytes;
+                if (coop_smem > coop_room && coop_smem <= prop.sharedMemPerBlockOptin) {
+                    coop_n = coop_warps = 0;
+                    coop_smem = 0;
+                }
+            }
         }
         SVG_CUDA(cudaMemcpyAsync(d_order, ord.data(), sizeof(int32_t) * (size_t)nsrc, cudaMemcpyHostToDevice, st));
         SVG_CUDA(cudaStreamSynchronize(st));
@@ -1473,15 +1487,11 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
             O.cand = b_cand.as<Cand>();
             O.cand_cap = cap;
             O.cand_start = b_candstart.as<int64_t>();
-            // the cooperative warps' heaps: window then pseudo-source entries
-            const size_t coop_smem =
-                coop_warps > 0 ? ((size_t)C.wstride * sizeof(HeapEntry) + (size_t)C.pstride * sizeof(HeapEntry)) : 0;
-            if (coop_smem > 48 * 1024)
+            if (coop_smem > 0)  // what a launch gets unasked, 48 KB, counts the lanes' state too
                 SVG_CUDA(cudaFuncSetAttribute(k_ich_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)coop_smem));
+                                              (int)std::max(coop_smem, coop_room)));
             k_ich_batched<<<blocks, tpb, coop_smem, st>>>(C, O);
             ++launches;
-            cap_coop_smem = coop_smem;
             cap_pool = cap;
             cap_attempts = attempt;
             SVG_CUDA(cudaGetLastError());
@@ -1637,7 +1647,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         P.O = O;
         P.blocks = blocks;
         P.tpb = tpb;
-        P.coop_smem = cap_coop_smem;
+        P.coop_smem = coop_smem;
         P.d_order = d_order;
         P.nsrc = nsrc;
         P.nv = nv;

@@ -126,6 +126,21 @@ def test_cooperative_form_matches_oracle_on_benchmark_mesh_samples(cfg, K, n):
     assert st["windows_generated"] == int(rows.stats[:, 0].sum())
 
 
+@pytest.mark.parametrize("cap,factor,coop", [(1472, 3, 100), (1473, 3, 100), (2047, 3, 100),
+                                             (12928, 26, 100), (12929, 26, 0)])
+def test_cooperative_heaps_of_every_size_are_built(cap, factor, coop):
+    """Cooperative heaps just within and beyond what a block gets unasked beside
+    the lanes' state (48 KB in all), the largest that can be asked for (227 KB in
+    all), and one entry more, which leaves the sources to the lanes: the rows of a
+    build without cooperative warps."""
+    pos, faces = meshgen.config_mesh(1, 0.3)
+    kw = dict(win_queue_cap=cap, heap_factor=factor, source_begin=0, source_end=300)
+    off, nodes, st, _, _ = coop_build(pos, faces, 500, coop_warps=8, coop_sources=100, **kw)
+    assert st["coop_sources"] == coop
+    want = gpu_build(pos, faces, 500, **kw)
+    assert compare_rows(off, nodes, want[0], want[1]) == []
+
+
 def test_automatic_cooperative_share_keeps_the_graph():
     """The automatic choice (heaviest sources above a lane's average share)
     gives the same CSR as a build with no cooperative warps."""
