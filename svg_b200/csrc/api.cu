@@ -623,6 +623,21 @@ svg_status svg_graph_set_query_form(svg_graph* g, int32_t form) {
     });
 }
 
+// Not part of the interface: for tests.  Limits of the waits of the whole-graph
+// searches that share all blocks of the GPU, in looks at the other blocks, while
+// they gather and at a barrier (0: no wait succeeds; negative: the library's
+// own).  *last (may be null): the latest launch of the graph's own queries, 1
+// all blocks gathered, 2 a wait ran out, 0 any other form.
+svg_status svg_test_query_waits(svg_graph* g, int32_t join_looks, int32_t barrier_looks, int32_t* last) {
+    return guarded([&]() -> svg_status {
+        if (!g) throw SvgError{SVG_ERR_ARG, "null graph"};
+        if (last) *last = query_last_form(g);
+        g->q_join_looks = join_looks;
+        g->q_barrier_looks = barrier_looks;
+        return SVG_OK;
+    });
+}
+
 svg_status svg_sssd_batch(svg_graph* g, int32_t n, const int32_t* s, const int32_t* t, double* dist) {
     return guarded([&]() -> svg_status {
         if (!g || n < 0 || (n > 0 && (!s || !t || !dist))) throw SvgError{SVG_ERR_ARG, "bad argument"};

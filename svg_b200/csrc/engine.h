@@ -117,6 +117,7 @@ struct svg_graph {
     double delta = 0.0;
     svg_qctx* qdefault = nullptr;
     int32_t qform = SVG_QUERY_CLUSTER;  // kernel form of the synchronous query calls
+    int32_t q_join_looks = -1, q_barrier_looks = -1;  // limits of the shared form's waits (tests; < 0: its own)
 };
 
 // Scratch of `slots` concurrent queries on one graph (see query.cu).
@@ -148,6 +149,7 @@ int query_slots_per_sm();            // plain form: query blocks resident per SM
 int query_cluster_size();            // cluster form: blocks per query
 int query_cluster_slots(int csize);  // cluster form: clusters resident at once
 void qctx_free(svg_qctx* c);
+int32_t query_last_form(svg_graph* g);  // kHeadState of the synchronous calls' last launch
 // parent pointers of n finished MSAD searches on the device (d_src may be null)
 void query_parents(svg_graph* g, int32_t n, const double* d_dist, const int32_t* d_src, int32_t* d_parent,
                    cudaStream_t st);

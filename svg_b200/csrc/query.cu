@@ -77,14 +77,15 @@ struct QParams {
     // grid form: blocks per query, and per query slot its counters and barrier
     int32_t group;
     QCtl* ctl;
-    int32_t fallback;      // cluster form: run only if the grid form before it did not
+    int32_t join_looks, barrier_looks;  // most looks at the others while gathering, and at a barrier
+    int32_t fallback;      // cluster form: run only if the grid form before it gave up
 };
-// Words of QParams::head; the first four are zeroed before every launch.
-//   kHeadNext    next query
-//   kHeadState   grid form: 0 gathering, 1 every block is there, 2 given up
-//   kHeadJoined  blocks there
-//   kHeadBroken  a barrier ran out: the context's slots are unusable
-enum { kHeadNext = 0, kHeadState = 1, kHeadJoined = 2, kHeadBroken = 8, kHeadZeroed = 4 };
+// Words of QParams::head, zeroed before every launch.
+//   kHeadNext       next query
+//   kHeadState      grid form: 0 gathering, 1 every block is there, 2 given up
+//   kHeadJoined     blocks there
+//   kHeadNextAgain  next query of the cluster form behind a grid form that gave up
+enum { kHeadNext = 0, kHeadState = 1, kHeadJoined = 2, kHeadNextAgain = 3, kHeadZeroed = 4 };
 
 __device__ __forceinline__ double hdist(const double* pos, int a, int b) {
     double dx = pos[3 * a] - pos[3 * b], dy = pos[3 * a + 1] - pos[3 * b + 1], dz = pos[3 * a + 2] - pos[3 * b + 2];
@@ -432,9 +433,9 @@ __device__ __forceinline__ DS ld_ds(const DS* p) {
 //                hold the GPU and some block has not come after a few
 //                milliseconds, all leave again before any query is begun, and
 //                the cluster form enqueued behind them serves the batch.  Once
-//                all are there they stay, so a barrier's wait is short; it gives
-//                up after kBarrierSpins looks (seconds), and the launch's
-//                unfinished queries and all later ones of the context report -1.
+//                all are there they stay, so a barrier's wait is short; where
+//                one runs out all the same (after kBarrierLooks looks, seconds),
+//                its team leaves, and the cluster form serves the batch again.
 struct ClusterTeam {
     QCtl* ctl;
     int size, rank, slot;
@@ -454,15 +455,14 @@ struct ClusterTeam {
         return true;
     }
 };
-constexpr int kBarrierSpins = 1 << 22;
-#ifndef SVG_JOIN_SPINS
-#define SVG_JOIN_SPINS (1 << 14)
-#endif
+constexpr int kBarrierLooks = 1 << 22;
+constexpr int kJoinLooks = 1 << 14;
 struct GridTeam {
     QCtl* ctl;
-    int size, rank, slot;
+    int size, rank, slot, looks;
     unsigned phase;
     __device__ GridTeam(const QParams& P, QCtl*) {
+        looks = P.barrier_looks;
         size = P.group;
         slot = (int)blockIdx.x / size;
         rank = (int)blockIdx.x % size;
@@ -473,9 +473,10 @@ struct GridTeam {
         int s = 0;
         if (threadIdx.x == 0) {
             int32_t* state = &P.head[kHeadState];
-            if (atomicAdd(&P.head[kHeadJoined], 1) + 1 == (int)gridDim.x) atomicCAS(state, 0, 1);
+            const int here = atomicAdd(&P.head[kHeadJoined], 1) + 1;
+            if (here == (int)gridDim.x && P.join_looks > 0) atomicCAS(state, 0, 1);
             for (int spins = 0; (s = *(volatile int32_t*)state) == 0; ++spins)
-                if (spins >= SVG_JOIN_SPINS) {
+                if (spins >= P.join_looks) {
                     s = atomicCAS(state, 0, 2);  // one word decides for all blocks
                     if (s == 0) s = 2;
                     break;
@@ -493,9 +494,8 @@ struct GridTeam {
             atomicAdd(&ctl->arrived, 1u);
             volatile unsigned* a = &ctl->arrived;
             int spins = 0;
-            while ((int)(*a - phase) < 0 && ++spins < kBarrierSpins) {
-            }
-            if (spins >= kBarrierSpins) atomicExch(&ctl->failed, 1);
+            while (spins < looks && (int)(*a - phase) < 0) ++spins;
+            if (spins >= looks) atomicExch(&ctl->failed, 1);
             __threadfence();
             ok = *(volatile int*)&ctl->failed ? 0 : 1;
         }
@@ -576,36 +576,26 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
         }
     };
 
-    // a barrier ran out in this launch or an earlier one: -1 for query q and
-    // all that no team has taken
-    auto give_up = [&](int q) {
-        if (tid == 0) atomicExch(&P.head[kHeadBroken], 1);
-        for (;;) {
-            if (q >= 0 && kSSSD && tid == 0) P.out[q] = -1.0;
-            if (q >= 0 && !kSSSD)
-                for (int v = tid; v < P.nv; v += kCThreads) P.out_dist[(size_t)q * P.nv + v] = -1.0;
-            __syncthreads();
-            if (tid == 0) s_base = atomicAdd(&P.head[kHeadNext], 1);
-            __syncthreads();
-            q = s_base;
-            if (q >= P.n) return;
+    // A barrier ran out: the launch has given up, and the slot's next query
+    // must not meet a stamp that this one's blocks have used.
+    uint32_t stamp = 0;
+    auto leave = [&]() {
+        if (tid == 0) {
+            atomicMax(&P.slot_stamp[team.slot], stamp);
+            atomicExch(&P.head[kHeadState], 2);
         }
     };
     if (!team.join(P)) return;
-    if (*(volatile int32_t*)&P.head[kHeadBroken]) {
-        give_up(-1);
-        return;
-    }
 
     for (;;) {
         if (leader) {
-            ctl->q = atomicAdd(&P.head[kHeadNext], 1);
+            ctl->q = atomicAdd(&P.head[P.fallback ? kHeadNextAgain : kHeadNext], 1);
             ctl->stamp = P.slot_stamp[team.slot];
         }
-        if (!team.sync()) return give_up(-1);
+        if (!team.sync()) return leave();
         const int q = *(volatile int*)&ctl->q;
-        uint32_t stamp = *(volatile uint32_t*)&ctl->stamp;
-        if (!team.sync()) return give_up(q < P.n ? q : -1);  // q and stamp read everywhere before the leader moves on (or any block leaves)
+        stamp = *(volatile uint32_t*)&ctl->stamp;
+        if (!team.sync()) return leave();  // q and stamp read everywhere before the leader moves on (or any block leaves)
         if (q >= P.n) break;
         const int tgt = kSSSD ? P.t[q] : -1;
 
@@ -627,7 +617,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 S.ds[v] = z;
             }
         }
-        if (!team.sync()) return give_up(q);
+        if (!team.sync()) return leave();
         stamp += 1;
         const uint32_t fst = stamp;
         if (kSSSD && leader) {
@@ -676,7 +666,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 ctl->init_far = nf;
             }
         }
-        if (!team.sync()) return give_up(q);
+        if (!team.sync()) return leave();
         int farN = *(volatile int*)&ctl->init_far;
         int32_t *far = S.far, *far2 = S.far2, *near = S.near, *next = S.next;
         long long rounds = 0;
@@ -741,7 +731,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 stage_flush(s_near, &ctl->nearA[ob], near, P.nv, &s_base);
                 stage_flush(s_far, &ctl->farB[ob], far2, P.list_cap, &s_base);
             }
-            if (!team.sync()) return give_up(q);
+            if (!team.sync()) return leave();
             {
                 int32_t* t = far; far = far2; far2 = t;
             }
@@ -846,7 +836,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                     stage_flush(s_near, &ctl->nextX[gb], next, P.nv, &s_base);
                     stage_flush(s_far, &ctl->farB[ob], far, P.list_cap, &s_base);
                 }
-                if (!team.sync()) return give_up(q);
+                if (!team.sync()) return leave();
                 nearN = *(volatile int*)&ctl->nextX[gb];
                 {
                     int32_t* t = near; near = next; next = t;
@@ -865,7 +855,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
                 const unsigned long long dt = __ldcg(&S.dist[tgt]);
                 P.out[q] = ovf ? -1.0 : (dt == kInfBits ? DBL_MAX : as_d(dt));
             }
-            if (!team.sync()) return give_up(q);  // the target's distance is read before the reset below
+            if (!team.sync()) return leave();  // the target's distance is read before the reset below
             const int tn = *(volatile int*)&ctl->touch;
             for (int i = gtid; i < tn; i += nthr) S.dist[__ldcg(&S.touched[i])] = kInfBits;
         } else {
@@ -878,7 +868,7 @@ __global__ void __launch_bounds__(kCThreads, SVG_QC_MINB) k_query_team(QParams P
             }
         }
         if (leader) P.slot_stamp[team.slot] = stamp;
-        if (!team.sync()) return give_up(q);
+        if (!team.sync()) return leave();
     }
 }
 
@@ -1178,8 +1168,18 @@ void fill_params(svg_qctx* c, QParams& P) {
     P.pos = g->mesh->d.pos;
     P.nv = g->nv;
     P.delta = g->delta;
+    P.join_looks = g->q_join_looks < 0 ? kJoinLooks : g->q_join_looks;
+    P.barrier_looks = g->q_barrier_looks < 0 ? kBarrierLooks : g->q_barrier_looks;
 }
 }  // namespace
+
+int32_t query_last_form(svg_graph* g) {
+    int32_t state = 0;
+    if (!g->qdefault) return state;
+    SVG_CUDA(cudaMemcpyAsync(&state, g->qdefault->head + kHeadState, sizeof(state), cudaMemcpyDeviceToHost, lib_stream()));
+    SVG_CUDA(cudaStreamSynchronize(lib_stream()));
+    return state;
+}
 
 void qctx_sssd(svg_qctx* c, int32_t n, const int32_t* d_s, const int32_t* d_t, double* d_dist, cudaStream_t st) {
     if (n <= 0) return;

@@ -231,3 +231,47 @@ def test_large_pair_batches_around_the_narrow_bucket_size(nu, nv):
     s.set_query_form(QUERY_PLAIN)
     assert np.array_equal(got, s.sssd_batch(S, T))
     s.set_query_form(QUERY_CLUSTER)
+
+
+@pytest.mark.parametrize("join,barrier", [(0, -1), (-1, 0), (-1, 1), (-1, 4), (-1, 16)])
+@pytest.mark.parametrize("n", [1, 5, 16])
+def test_waits_that_run_out_leave_the_search_to_clusters(n, join, barrier):
+    """Teams of all blocks whose gathering, or whose first or some later barrier,
+    runs out after a few looks: the plain form's distances, sources that explain
+    them, parents, and a graph whose next calls use the teams again."""
+    import ctypes as C
+    from svg_b200 import QUERY_CLUSTER, QUERY_PLAIN, lib
+    waits = lib().svg_test_query_waits
+    waits.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]
+    pos, faces = meshgen.torus(1.0, 0.35, 120, 90, 0.02, seed=16)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    s.ConstructSVG(with_paths=False)
+    rng = np.random.default_rng(n)
+    sets = [rng.choice(m.vertNum, int(k), replace=False).astype(np.int32) for k in rng.integers(1, 40, n)]
+    weights = [rng.uniform(0, 0.2, len(x)) for x in sets]
+    s.set_query_form(QUERY_PLAIN)
+    want, _, parents = s.msad_paths(sets, weights)
+    s.set_query_form(QUERY_CLUSTER)
+
+    def check(join_looks, barrier_looks):
+        last = C.c_int32()
+        assert waits(s._g, join_looks, barrier_looks, None) == 0
+        d, src = s.msad_batch(sets, weights)
+        assert waits(s._g, -1, -1, C.byref(last)) == 0
+        assert np.array_equal(d, want)
+        for q in range(n):
+            reached = d[q] < DBL_MAX
+            assert np.isin(src[q][reached], sets[q]).all() and np.all(src[q][~reached] == -1)
+        return last.value
+
+    assert check(-1, -1) == 1
+    for _ in range(3):
+        last = check(join, barrier)
+        assert last == 2 if 0 in (join, barrier) else last in (1, 2)
+    assert check(-1, -1) == 1
+    assert waits(s._g, join, barrier, None) == 0
+    pd, ps, par = s.msad_paths(sets, weights)
+    assert np.array_equal(pd, want) and (par == parents).mean() > 0.999
