@@ -430,9 +430,9 @@ __device__ __forceinline__ DS ld_ds(const DS* p) {
 //   GridTeam     any number of blocks of a launch no larger than the GPU holds:
 //                counters in global memory and a barrier on one of them.  The
 //                blocks of the launch first gather (join): where other streams
-//                hold the GPU and some block has not come after a few
-//                milliseconds, all leave again before any query is begun, and
-//                the cluster form enqueued behind them serves the batch.  Once
+//                hold the GPU and some block has not come after kJoinLooks
+//                looks, all leave again before any query is begun, and the
+//                cluster form enqueued behind them serves the batch.  Once
 //                all are there they stay, so a barrier's wait is short; where
 //                one runs out all the same (after kBarrierLooks looks, seconds),
 //                its team leaves, and the cluster form serves the batch again.
@@ -456,7 +456,12 @@ struct ClusterTeam {
     }
 };
 constexpr int kBarrierLooks = 1 << 22;
-constexpr int kJoinLooks = 1 << 14;
+// Gathering that fails costs its looks on every call: 0.16 ms for 1,024 of them,
+// 2.5 ms for 16,384 (one search on 120K vertices beside a kernel of another
+// stream, 3.24 ms by clusters alone).  On a free GPU the blocks gather within 16
+// looks, between 4096^3 matrix products of another stream within 512 (with 256,
+// 18 of 60 calls did).
+constexpr int kJoinLooks = 1 << 10;
 struct GridTeam {
     QCtl* ctl;
     int size, rank, slot, looks;

@@ -275,3 +275,39 @@ def test_waits_that_run_out_leave_the_search_to_clusters(n, join, barrier):
     assert waits(s._g, join, barrier, None) == 0
     pd, ps, par = s.msad_paths(sets, weights)
     assert np.array_equal(pd, want) and (par == parents).mean() > 0.999
+
+
+def test_a_gathering_that_fails_is_short():
+    """Beside a kernel of another stream that holds part of one SM, the blocks of
+    a whole-graph search cannot all gather: the wait before the clusters take
+    over stays well below a millisecond."""
+    import ctypes as C
+    import time
+
+    import torch
+    from svg_b200 import lib
+    waits = lib().svg_test_query_waits
+    waits.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.POINTER(C.c_int32)]
+    pos, faces = meshgen.torus(1.0, 0.35, 400, 300, 0.02, seed=16)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    s.ConstructSVG(with_paths=False)
+    other = torch.cuda.Stream()
+
+    def call(join_looks):
+        times, last = [], C.c_int32()
+        for _ in range(9):
+            assert waits(s._g, join_looks, -1, None) == 0
+            with torch.cuda.stream(other):
+                torch.cuda._sleep(60_000_000)
+            t = time.perf_counter()
+            s.msad_batch([[5, 70000]])
+            times.append(time.perf_counter() - t)
+            assert waits(s._g, -1, -1, C.byref(last)) == 0 and last.value == 2
+            torch.cuda.synchronize()
+        return np.median(times) * 1e3
+
+    call(0)
+    assert call(-1) - call(0) < 1.0
