@@ -116,6 +116,7 @@ struct svg_graph {
     // the synchronous batch entry points
     double delta = 0.0;
     svg_qctx* qdefault = nullptr;
+    bool qsmall_failed = false;  // no room for the context of large pair batches
     int32_t qform = SVG_QUERY_CLUSTER;  // kernel form of the synchronous query calls
     int32_t q_join_looks = -1, q_barrier_looks = -1;  // limits of the shared form's waits (tests; < 0: its own)
 };

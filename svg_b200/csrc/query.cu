@@ -1093,14 +1093,20 @@ constexpr size_t kSmallTeamBytes = (size_t)4 << 30;  // most scratch of a contex
 // a quarter 25.8 on 73K and 125 on 750K.  A single pair 0.28 / 0.31 on 30K.
 constexpr int kNarrowVertices = 30000;
 
+// The fewest slots with which 4-block clusters are used: with less of the GPU
+// than 8-block ones fill they are slower.  300 / 2,048 pairs on the 750K torus,
+// 8-block clusters 47 / 258 ms; 4-block ones in 38 slots 66 / 340, 52 55 / 262, 58
+// 51 / 240, 64 50 / 222, 70 47 / 207, all of them 47 / 205.
+int small_team_slots() { return (7 * query_cluster_slots(kSmallTeam) + 7) / 8; }
+
 // Cluster size of one call: a context made with `adaptive` serves a batch that
 // fits in the resident clusters of its size at that size (latency), and a
 // larger batch with 8-block clusters, which pack the SMs more fully
 // (throughput), or 4-block ones (large single-pair batches, where the context
-// has slots for them); otherwise the context's own size.
+// has slots enough for them); otherwise the context's own size.
 int call_cluster(const svg_qctx* c, int n, bool sssd) {
     if (!c->adaptive || c->cluster <= 8 || n <= query_cluster_slots(c->cluster)) return c->cluster;
-    return sssd && n >= kSmallTeamQueries && c->slots > query_cluster_slots(8) ? kSmallTeam : 8;
+    return sssd && n >= kSmallTeamQueries && c->slots >= small_team_slots() ? kSmallTeam : 8;
 }
 }  // namespace
 
@@ -1253,7 +1259,8 @@ namespace {
 // The graph's own context for the synchronous batch entry points: as many
 // clusters as run at once (cluster form), or every resident block (plain form).
 // A large single-pair batch replaces a cluster context by one with slots for
-// 4-block clusters, within kSmallTeamBytes.
+// 4-block clusters, where enough of those take at most kSmallTeamBytes and the
+// device has the room; otherwise the context stays, and 8-block clusters serve the batch.
 svg_qctx* default_ctx(svg_graph* g, bool small_teams) {
     if (g->qform == SVG_QUERY_PLAIN) {
         if (!g->qdefault) {
@@ -1264,19 +1271,27 @@ svg_qctx* default_ctx(svg_graph* g, bool small_teams) {
         }
         return g->qdefault;
     }
-    const int cs = query_cluster_size();
-    int slots = std::max(query_cluster_slots(cs), query_cluster_slots(8));
-    if (small_teams)
-        slots = (int)std::max<size_t>((size_t)slots, std::min((size_t)query_cluster_slots(kSmallTeam),
-                                                              kSmallTeamBytes / std::max<size_t>(slot_size(g->nv), 1)));
-    if (g->qdefault && g->qdefault->slots < slots) {
-        SVG_CUDA(cudaStreamSynchronize(lib_stream()));
-        qctx_free(g->qdefault);
-        g->qdefault = nullptr;
+    const int cs = query_cluster_size(), usual = std::max(query_cluster_slots(cs), query_cluster_slots(8));
+    int slots = usual;
+    if (small_teams && !g->qsmall_failed) {
+        const int small = (int)std::min((size_t)query_cluster_slots(kSmallTeam), kSmallTeamBytes / slot_size(g->nv));
+        if (small >= small_team_slots()) slots = std::max(slots, small);
     }
-    if (!g->qdefault) {
-        g->qdefault = qctx_create(g, slots, lib_stream(), cs);
-        g->qdefault->adaptive = true;
+    if (!g->qdefault || g->qdefault->slots < slots) {
+        svg_qctx* c = nullptr;
+        try {
+            c = qctx_create(g, slots, lib_stream(), cs);
+        } catch (const SvgError& e) {
+            if (e.code != SVG_ERR_NOMEM || slots == usual) throw;
+            g->qsmall_failed = true;  // a failed allocation empties the cache of device blocks: not at every call
+            if (!g->qdefault) c = qctx_create(g, usual, lib_stream(), cs);
+        }
+        if (c) {
+            SVG_CUDA(cudaStreamSynchronize(lib_stream()));
+            qctx_free(g->qdefault);
+            g->qdefault = c;
+            c->adaptive = true;
+        }
     }
     return g->qdefault;
 }

@@ -311,3 +311,44 @@ def test_a_gathering_that_fails_is_short():
 
     call(0)
     assert call(-1) - call(0) < 1.0
+
+
+@pytest.mark.parametrize("before", [True, False])
+def test_large_pair_batches_without_room_for_a_larger_context(before):
+    """300 pairs where the device has room for the usual query context (0.6 GB)
+    or, with that made before, for nothing more, but not for the larger one
+    (1.3 GB): served as before, and so are the calls after them."""
+    import gc
+
+    import torch
+
+    from svg_b200 import lib
+    gc.collect()   # graphs of earlier tests: no blocks of theirs return in between
+    pos, faces = meshgen.torus(1.0, 0.35, 600, 500, 0.02, seed=17)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(10)
+    s.ConstructSVG(with_paths=False)
+    rng = np.random.default_rng(0)
+    S, T = rng.integers(0, m.vertNum, (2, 300)).astype(np.int32)
+    if before:
+        few = s.sssd_batch(S[:3], T[:3])
+    lib().svg_trim_device_cache()
+    torch.cuda.empty_cache()
+    left = (300 if before else 1000) << 20
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+    try:
+        got = s.sssd_batch(S, T)
+        again = s.sssd_batch(S, T)
+        if before:
+            assert np.array_equal(few, got[:3])
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    s2 = SVG()
+    s2.AssignMesh(m)
+    s2.SetParameters(10)
+    s2.ConstructSVG(with_paths=False)
+    want = s2.sssd_batch(S, T)
+    assert np.array_equal(got, want) and np.array_equal(again, want)
