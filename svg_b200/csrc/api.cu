@@ -245,6 +245,24 @@ __global__ void __launch_bounds__(256) k_pack_nodes(const int32_t* __restrict__ 
     }
 }
 
+// What k_pack_nodes does, for edges [first, first + n), without device memory.
+void host_nodes(const svg_graph* g, int64_t first, int64_t n, svg_node* nodes) {
+    std::vector<int32_t> adj((size_t)n);
+    std::vector<double> dist((size_t)n);
+    std::vector<PathEnd> pe((size_t)n, PathEnd{0xFFFFFFFFu, 0xFFFFFFFFu, 0.0, 0.0});
+    cudaStream_t st = lib_stream();
+    SVG_CUDA(cudaMemcpyAsync(adj.data(), g->adj + first, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost, st));
+    SVG_CUDA(cudaMemcpyAsync(dist.data(), g->dist + first, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, st));
+    if (g->with_paths)
+        SVG_CUDA(cudaMemcpyAsync(pe.data(), static_cast<const PathEnd*>(g->paths) + first, sizeof(PathEnd) * (size_t)n,
+                                 cudaMemcpyDeviceToHost, st));
+    SVG_CUDA(cudaStreamSynchronize(st));
+    for (int64_t i = 0; i < n; ++i) {
+        const PathEnd& p = pe[(size_t)i];
+        nodes[i] = svg_node{adj[(size_t)i], 0, dist[(size_t)i], p.src_edge, p.dst_edge, p.src_x, p.dst_x};
+    }
+}
+
 }  // namespace svgb
 
 using namespace svgb;
@@ -475,13 +493,23 @@ svg_status svg_graph_copy_nodes(const svg_graph* g, int32_t* tails, svg_node* no
         }
         if (nodes && g->nnz) {
             static_assert(sizeof(svg_node) == 40, "k_pack_nodes writes five words a node");
-            // assembled on the device, a bounded piece at a time
-            constexpr int64_t kPiece = (int64_t)8 << 20;  // nodes: 320 MB
+            // assembled on the device, a bounded piece at a time, or, with no
+            // room for a piece there, from the three arrays on the host
+            constexpr int64_t kPiece = (int64_t)1 << 20;  // nodes: 40 MB
             const int64_t piece = std::min<int64_t>(g->nnz, kPiece);
             DevBuf b;
-            b.reserve(sizeof(svg_node) * (size_t)piece);
+            bool room = true;
+            try {
+                b.reserve(sizeof(svg_node) * (size_t)piece);
+            } catch (const SvgError&) {
+                room = false;
+            }
             for (int64_t first = 0; first < g->nnz; first += piece) {
                 const int64_t n = std::min(piece, g->nnz - first);
+                if (!room) {
+                    host_nodes(g, first, n, nodes + first);
+                    continue;
+                }
                 k_pack_nodes<<<(int)std::min<int64_t>((5 * n + 255) / 256, 4736), 256, 0, st>>>(
                     g->adj, g->dist, g->with_paths ? static_cast<const PathEnd*>(g->paths) : nullptr, first, n,
                     b.as<unsigned long long>());

@@ -367,3 +367,31 @@ def test_emission_of_short_and_long_candidate_lists(K):
     out = [gpu_build(pos, faces, K, mode, source_begin=1500, source_end=1540)[:2] for mode in (MODE_BATCHED, MODE_PLAIN)]
     assert np.diff(out[0][0]).max() == K
     assert compare_rows(*out[0], *out[1]) == []
+
+
+@pytest.mark.parametrize("with_paths", [True, False])
+def test_rows_reach_the_host_without_device_memory(with_paths):
+    """With 8 MB of the device left (a piece of the rows takes 20), the nodes are
+    assembled on the host: the same rows, padding included, and the same file."""
+    import gc
+
+    import torch
+
+    import svg_b200
+    pos, faces = meshgen.torus(1.0, 0.35, 130, 100, 0.02, seed=5)
+    off, nodes, _, s, _ = gpu_build(pos, faces, 40, with_paths=with_paths)
+    assert 40 * len(nodes) > 16 << 20
+    with tempfile.TemporaryDirectory() as td:
+        s.SaveSVGToFile(os.path.join(td, "a"))
+        gc.collect()
+        svg_b200.lib().svg_trim_device_cache()
+        torch.cuda.empty_cache()
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (8 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            off2, nodes2 = s.CopySVGToHost()
+            s.SaveSVGToFile(os.path.join(td, "b"))
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        a, b = (open(os.path.join(td, x), "rb").read() for x in "ab")
+    assert np.array_equal(off, off2) and nodes.tobytes() == nodes2.tobytes() and a == b
