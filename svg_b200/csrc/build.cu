@@ -1280,9 +1280,12 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         // flight, at large K.  Full / equal waves: 73K torus K = 100 29.0 /
         // 28.0 ms, K = 500 288 / 268 ms, 120K K = 200 125 / 117 ms; 73K height
         // field K = 500 438 / 411 ms, but K = 100 26.2 / 28.7 ms and 120K
-        // K = 200 134 / 141 ms.
+        // K = 200 134 / 141 ms.  A launch of up to two blocks per SM (the
+        // caller's number, as a server's builds beside queries) wants every
+        // lane: K = 500, 40K height field at one 424 / 517 ms, at two 300 /
+        // 347 ms, 30K torus at one and a half 213 / 244 ms.
         const int64_t warps = (int64_t)blocks * (tpb / 32);
-        const bool equal = K >= 300 || (m->cost_K == K && m->cost_even);
+        const bool equal = warps > 8 * prop.multiProcessorCount && (K >= 300 || (m->cost_K == K && m->cost_even));
         const int64_t waves = equal ? std::max<int64_t>(1, (nsrc + 32 * warps - 1) / (32 * warps)) : 1;
         warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps * waves - 1) / (warps * waves)));
         const int64_t per_block = (int64_t)(tpb / 32) * warp_lanes;

@@ -395,3 +395,19 @@ def test_rows_reach_the_host_without_device_memory(with_paths):
             torch.cuda.empty_cache()
         a, b = (open(os.path.join(td, x), "rb").read() for x in "ab")
     assert np.array_equal(off, off2) and nodes.tobytes() == nodes2.tobytes() and a == b
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 5])
+def test_a_small_launch_uses_every_lane(blocks):
+    """At K = 300 launches of the whole GPU make their waves equal by using fewer
+    lanes of each warp; one of few blocks with one source more than its lanes
+    keeps them all (the same scratch), and its rows."""
+    pos, faces = meshgen.config_mesh(1, 0.2)
+    lanes, scratch, rows = 128 * blocks, [], []
+    for n in (lanes, lanes + 1):
+        off, nodes, st, _, _ = gpu_build(pos, faces, 300, blocks=blocks, heavy_first=0, source_begin=0, source_end=n)
+        scratch.append(st["scratch_bytes"])
+        rows.append((off, nodes))
+    assert scratch[0] == scratch[1]
+    want = gpu_build(pos, faces, 300, source_begin=0, source_end=lanes + 1)
+    assert compare_rows(*rows[1], *want[:2]) == []
