@@ -1374,13 +1374,19 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         if (o.coop_sources > 0 || (o.coop_sources < 0 && !m->cost_probe)) {
             double total = 0.0;
             for (int32_t i = 0; i < nsrc; ++i) total += (double)cost[(size_t)(sb + i)];
-            const double share = total / (double)lay.lanes;
+            // (the share of a lane at two blocks per SM: at three there is nearly a
+            // lane for every source of the meshes this is used on, every second
+            // source is above the share, and the warps that run them are missed
+            // elsewhere: 73K height field K = 200 110.7 ms with 888 of them, 92K
+            // 123 with 711)
+            const int64_t share_lanes = std::min<int64_t>(lay.lanes, 2 * prop.multiProcessorCount * 128);
+            const double share = total / (double)share_lanes;
             int64_t n = 0;
             if (o.coop_sources > 0) {
                 n = std::min<int64_t>(o.coop_sources, nsrc);
             } else {
                 while (n < head && (double)cost[(size_t)ord[(size_t)n]] >= share) ++n;
-                n = std::min<int64_t>(n, lay.lanes / 64);
+                n = std::min<int64_t>(n, share_lanes / 64);
             }
             const int64_t warps = (int64_t)blocks * (tpb / 32);
             coop_n = (int32_t)n;
@@ -1401,6 +1407,12 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
                     coop_n = coop_warps = 0;
                     coop_smem = 0;
                 }
+            }
+            // the others' first wave strided over the warps that begin with them
+            const int64_t begin = warps - coop_warps, wave = begin * warp_lanes;
+            if (wave <= nsrc - coop_n) {
+                const std::vector<int32_t> front(ord.begin() + coop_n, ord.begin() + coop_n + wave);
+                for (int64_t i = 0; i < wave; ++i) ord[(size_t)(coop_n + i)] = front[(size_t)strided(i, begin, warp_lanes)];
             }
         }
         SVG_CUDA(cudaMemcpyAsync(d_order, ord.data(), sizeof(int32_t) * (size_t)nsrc, cudaMemcpyHostToDevice, st));

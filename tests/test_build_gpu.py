@@ -411,3 +411,23 @@ def test_a_small_launch_uses_every_lane(blocks):
     assert scratch[0] == scratch[1]
     want = gpu_build(pos, faces, 300, source_begin=0, source_end=lanes + 1)
     assert compare_rows(*rows[1], *want[:2]) == []
+
+
+def test_automatic_cooperative_share_counts_two_blocks_per_sm():
+    """The sources that cost more than a lane's average share of the build are
+    counted with the lanes of two blocks per SM, also where three run, and their
+    rows stay."""
+    import torch
+    pos, faces = meshgen.config_mesh(1)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(50)
+    s.ConstructSVG(heavy_first=0)
+    want = s.csr()
+    cost = s.source_stats()[0].astype(np.int64)
+    st = s.ConstructSVG(heavy_first=1, coop_sources=-1)
+    lanes = 2 * torch.cuda.get_device_properties(0).multi_processor_count * 128
+    assert st["coop_sources"] == min((cost >= cost.sum() / lanes).sum(), lanes // 64)
+    for x, y in zip(want, s.csr()):
+        assert np.array_equal(x, y)
