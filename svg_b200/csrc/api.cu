@@ -76,8 +76,8 @@ void* dev_alloc(size_t bytes) {
         e = cudaMalloc(&q, n);
         if (e != cudaSuccess) {
             cudaGetLastError();
-            throw SvgError{SVG_ERR_NOMEM, "device allocation of " + std::to_string(n) + " bytes failed: " +
-                                              cudaGetErrorString(e)};
+            throw DevNoMem{{SVG_ERR_NOMEM, "device allocation of " + std::to_string(n) + " bytes failed: " +
+                                               cudaGetErrorString(e)}};
         }
     }
     std::lock_guard<std::mutex> lk(P.mu);

@@ -1144,7 +1144,9 @@ void capture_graph(svg_mesh* m, const svg_build_opts& o, const CapturePlan& P, s
 }
 }  // namespace
 
-svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
+namespace {
+// A build whose launch, where it chooses one, has at most `most_per_sm` blocks per SM.
+svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int most_per_sm) {
     const svg_build_opts o = effective_options(m, o_in);
     upload_mesh(m);
     if (o.graph && o.mode != SVG_BUILD_PLAIN && replay_graph(m, o, g)) return SVG_OK;
@@ -1262,7 +1264,7 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         // From there three are as fast or faster: 30K torus K = 100 13.9 / 13.5
         // ms, 73K height field K = 500 441 / 411 ms, 750K torus 271 / 229 ms.
         if (per_sm > 2 && nsrc <= 8 * 2 * prop.multiProcessorCount * (tpb / 32)) per_sm = 2;
-        blocks = std::max(1, per_sm) * prop.multiProcessorCount;
+        blocks = std::max(1, std::min(per_sm, most_per_sm)) * prop.multiProcessorCount;
     }
     // Active lanes per warp.  Fewer sources than lanes: every warp gets as few
     // of them as spreads them over all warps.  A warp's step waits for its slowest lane and runs every
@@ -1686,6 +1688,22 @@ svg_status run_build(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g) {
         capture_graph(m, o, P, g);
     }
     return SVG_OK;
+}
+}  // namespace
+
+// The third block per SM takes half as much scratch again.  A build that finds
+// no room for its candidates or its rows beside it (a mesh of some ten sources
+// per lane or more, on a nearly full device) is run again with two.
+svg_status run_build(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
+    try {
+        return build_once(m, o, g, INT32_MAX);
+    } catch (const DevNoMem&) {
+        if (o.mode == SVG_BUILD_PLAIN || o.blocks > 0) throw;
+    }
+    free_graph_device(g);
+    for (Arena& a : g_arena) a.buf.release();
+    dev_trim();  // the budget is taken from what the device has free
+    return build_once(m, o, g, 2);
 }
 
 // ------------------------------------------------------------ autotuner

@@ -32,6 +32,9 @@ struct SvgError {
     std::string msg;
 };
 
+// Device memory ran out (dev_alloc), as against a limit of the library's own.
+struct DevNoMem : SvgError {};
+
 // The library's CUDA stream and events (one device: the current one at first use).
 cudaStream_t lib_stream();
 

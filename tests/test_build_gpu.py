@@ -431,3 +431,39 @@ def test_automatic_cooperative_share_counts_two_blocks_per_sm():
     assert st["coop_sources"] == min((cost >= cost.sum() / lanes).sum(), lanes // 64)
     for x, y in zip(want, s.csr()):
         assert np.array_equal(x, y)
+
+
+_NEARLY_FULL = """
+import sys
+import numpy as np, torch
+from svg_b200 import SVG, Mesh, meshgen
+pos, faces = meshgen.torus(1.0, 0.35, 1250, 800, 0.0, seed=1)
+m = Mesh.from_arrays(pos, faces)
+m.copyToGPU()
+s = SVG()
+s.AssignMesh(m)
+s.SetParameters(10)
+torch.empty(1, device="cuda")
+hold = torch.empty(torch.cuda.mem_get_info()[0] - (3640 << 20), dtype=torch.uint8, device="cuda")
+st = s.ConstructSVG()
+got = s.csr()
+print("scratch", st["scratch_bytes"])
+del hold
+torch.cuda.empty_cache()
+want_st = s.ConstructSVG(blocks=2 * torch.cuda.get_device_properties(0).multi_processor_count)
+assert st["scratch_bytes"] == want_st["scratch_bytes"]
+assert all(np.array_equal(x, y) for x, y in zip(got, s.csr()))
+"""
+
+
+def test_a_build_without_room_for_three_blocks_per_sm_runs_two():
+    """1 M sources at K = 10 with 3.6 GB of the device left: the scratch of three
+    blocks per SM (1.8 GB, half of that) leaves no room for the candidates and
+    rows, that of two does, as when two were all there were.  In a process of its
+    own: scratch that an earlier build left would count."""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _NEARLY_FULL], cwd=root, env=dict(os.environ, PYTHONPATH=root),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
