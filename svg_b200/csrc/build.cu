@@ -758,7 +758,8 @@ Arena g_arena[2];  // [0] main pass, [1] retry pass with larger tables
 // stream behind it: streams share the GPU's few hardware queues, and a copy
 // that waits for a long build holds up the queries of every stream that shares
 // its queue.  Queries of a server beside a build, p99: 300K vertices K = 200
-// 577 -> 2.6 ms (it was the build's length), 150K 317 -> 2.8.
+// 577 -> 2.6 ms (it was the build's length), 150K 317 -> 2.8.  (A replayed
+// graph's own nodes wait behind its build kernel all the same.)
 void wait_idle(cudaStream_t st) {
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
@@ -1540,9 +1541,16 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
                 C2.scap_log2 = l2.scap_log2;
                 C2.vlimit = l2.vlimit;
                 C2.slimit = (int32_t)(((int64_t)3 << l2.scap_log2) / 4);
-                // spread over the warps as in the first pass
+                // spread over the warps as in the first pass; a caller's number of
+                // blocks (room for queries beside the build) holds here too, unless
+                // full warps need more.  14K sources of a 40K height field at K = 500
+                // on all SMs, the build one block per SM: 277 -> 310 ms, a query
+                // beside it at most 152 -> 0.5 ms
                 const int tb2 = 64;
                 int bl2 = prop.multiProcessorCount * 4;
+                if (o.blocks > 0)
+                    bl2 = (int)std::min<int64_t>(bl2, std::max<int64_t>(((int64_t)o.blocks * tpb + tb2 - 1) / tb2,
+                                                                        ((int64_t)retry_n + tb2 - 1) / tb2));
                 const int wl2 = (int)std::min<int64_t>(32, ((int64_t)retry_n + 2 * bl2 - 1) / (2 * bl2));
                 bl2 = (int)std::min<int64_t>(bl2, ((int64_t)retry_n + 2 * wl2 - 1) / (2 * wl2));
                 l2.lanes = bl2 * 2 * wl2;
@@ -1565,6 +1573,7 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
                 k_ich_batched<<<bl2, tb2, 0, st>>>(C2, O2);
                 ++launches;
                 SVG_CUDA(cudaGetLastError());
+                wait_idle(st);
                 int32_t again = 0;
                 SVG_CUDA(cudaMemcpyAsync(&again, d_work + 3, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
                 read_lists();

@@ -195,3 +195,53 @@ def test_msad_results_into_caller_buffers(graph):
     for q, (bd, bs) in enumerate(bufs):
         assert np.array_equal(bd, d[q])
         assert (bs == src[q]).mean() > 0.999
+
+
+_BESIDE = """
+import sys, threading, time
+import numpy as np
+from svg_b200 import SVG, Mesh, Server, meshgen
+g = SVG()
+g.AssignMesh(Mesh.from_arrays(*meshgen.torus(1.0, 0.35, 100, 50, 0.02, seed=9)))
+g.SetParameters(50)
+g.ConstructSVG(with_paths=False)
+srv = Server()
+gid = srv.add_graph(g)
+m = Mesh.from_arrays(*meshgen.height_field(200, seed=7))
+m.copyToGPU()
+s = SVG()
+s.AssignMesh(m)
+s.SetParameters(500)
+kw = dict(blocks=148, source_begin=0, source_end=15000, heap_factor=int(sys.argv[1]))
+for run in range(2):
+    took = []
+    def build():
+        t = time.perf_counter()
+        took.append(s.ConstructSVG(**kw))
+        took.append(time.perf_counter() - t)
+    th = threading.Thread(target=build)
+    th.start()
+    worst = 0.0
+    while th.is_alive():
+        t = time.perf_counter()
+        srv.wait(srv.submit_sssd(gid, 3, 2500))
+        worst = max(worst, time.perf_counter() - t)
+        time.sleep(0.001)
+    th.join()
+assert (took[0]["retried_sources"] > 5000) == (kw["heap_factor"] == 1), took
+assert took[1] > 0.1 and worst < 0.25 * took[1], (took[1], worst)
+"""
+
+
+@pytest.mark.parametrize("heap_factor", [3, 1])
+def test_queries_do_not_wait_for_a_build_beside_them(heap_factor):
+    """With one hardware queue for all streams, whatever waits on the stream
+    behind a running build kernel holds up every query: a build of one block per
+    SM, without and with a long retry pass, lets them through."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _BESIDE, str(heap_factor)], cwd=root, capture_output=True, text=True,
+                       env=dict(os.environ, PYTHONPATH=root, CUDA_DEVICE_MAX_CONNECTIONS="1"), timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
