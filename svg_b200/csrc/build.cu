@@ -993,8 +993,8 @@ bool replay_graph(svg_mesh* m, const svg_build_opts& o, svg_graph* g) {
     S.ms_total = ms;
     S.edges = nnz;
     S.sources = bg->nsrc;
-    S.launches = (SVG_SPLIT_TRACE && bg->opts.with_paths) ? 4 : 3;  // k_ich_batched, the offsets scan,
-                                                                     // k_emit (and k_trace), in one graph launch
+    S.launches = (SVG_SPLIT_TRACE && bg->opts.with_paths) ? 5 : 4;  // k_ich_batched, the offsets scan, k_emit
+                                                                     // (and k_trace) in one graph launch; k_tally
     S.scratch_bytes = bg->scratch_bytes;
     S.coop_sources = bg->coop_n;
     S.coop_warps = bg->coop_warps;
@@ -1316,6 +1316,7 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
     b_order.reserve(sizeof(int32_t) * (size_t)std::max(nsrc, 1));
     int32_t* d_order = b_order.as<int32_t>();
     bool ordered = false;
+    int launches = 0;
     const bool one_wave = nsrc <= lay.lanes;
     const int32_t wave_warps = plain ? 0 : std::min(nsrc, lay.lanes) / warp_lanes;
     // The heaviest sources, two per lane, go first (they would otherwise
@@ -1348,6 +1349,7 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
         k_cost_plan<<<1, 1024, 0, st>>>(P);
         k_cost_scatter<<<(nsrc + 255) / 256, 256, 0, st>>>(P);
         SVG_CUDA(cudaGetLastError());
+        launches += 3;
         ordered = true;
     } else if (by_cost && o.coop_sources != 0) {
         // the cooperative warps take their sources from the front, in cost order
@@ -1422,8 +1424,10 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
         SVG_CUDA(cudaStreamSynchronize(st));
         ordered = true;
     }
-    if (nsrc > 0 && !ordered)
+    if (nsrc > 0 && !ordered) {
         k_order<<<(nsrc + 255) / 256, 256, 0, st>>>(d_order, nsrc, sb, wave_warps, warp_lanes);
+        ++launches;
+    }
     // misc: work, retry_n, acc[8], cand_used ; retry list ; cand_n ; deg
     // retry list: room for the first pass's failures and, after them, the retry pass's
     size_t retry_bytes = align_up(sizeof(int32_t) * 2 * (size_t)std::max(nsrc, 1));
@@ -1468,7 +1472,6 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
 
     cudaEvent_t ev[4];
     for (auto& e : ev) SVG_CUDA(cudaEventCreate(&e));
-    int launches = 1;  // the work order
     SVG_CUDA(cudaEventRecord(ev[0], st));
 
     DevBuf b_padj, b_pdist, b_ppath, b_tails;
@@ -1662,7 +1665,7 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
     S.edges = nnz;
     S.sources = nsrc;
     S.retried_sources = retry_n;
-    S.launches = launches;
+    S.launches = launches + 1;  // k_tally
     S.scratch_bytes = scratch_bytes;
     S.coop_sources = coop_n;
     S.coop_warps = coop_warps;

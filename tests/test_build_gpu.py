@@ -467,3 +467,25 @@ def test_a_build_without_room_for_three_blocks_per_sm_runs_two():
     r = subprocess.run([sys.executable, "-c", _NEARLY_FULL], cwd=root, env=dict(os.environ, PYTHONPATH=root),
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_launches_are_counted():
+    """Work order (one kernel, three by cost, none for the host's), search, offsets
+    scan, emission, path ends and flag tallies; plain: rows packed instead of
+    emitted; replayed: no order."""
+    pos, faces = meshgen.torus(1.0, 0.35, 30, 20, 0.02, seed=5)
+    m = Mesh.from_arrays(pos, faces)
+    s = SVG()
+    s.AssignMesh(m)
+    s.SetParameters(20)
+    assert s.ConstructSVG()["launches"] == 6
+    assert s.ConstructSVG(with_paths=False)["launches"] == 5
+    assert s.ConstructSVG(mode=MODE_PLAIN)["launches"] == 5
+    one = dict(blocks=1, threads_per_block=32, heavy_first=1)   # more sources than lanes
+    uneven = dict(one, source_begin=0, source_end=60)           # fewer than 3.5 waves: by cost
+    s.ConstructSVG(**uneven)
+    assert s.ConstructSVG(**uneven)["launches"] == 8
+    assert s.ConstructSVG(**uneven, coop_sources=2)["launches"] == 5
+    s.ConstructSVG(graph=1)
+    st = s.ConstructSVG(graph=1)
+    assert st["graph_replayed"] == 1 and st["launches"] == 5
