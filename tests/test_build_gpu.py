@@ -489,3 +489,13 @@ def test_launches_are_counted():
     s.ConstructSVG(graph=1)
     st = s.ConstructSVG(graph=1)
     assert st["graph_replayed"] == 1 and st["launches"] == 5
+
+
+def test_three_blocks_of_the_build_kernel_run_per_sm():
+    """A build of many sources launches three blocks per SM (its registers just
+    allow it): the scratch of as many blocks asked for."""
+    import torch
+    pos, faces = meshgen.torus(1.0, 0.35, 300, 200, 0.02, seed=5)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    a = gpu_build(pos, faces, 10, heavy_first=0)[2]["scratch_bytes"]
+    assert a == gpu_build(pos, faces, 10, heavy_first=0, blocks=3 * sms)[2]["scratch_bytes"]
