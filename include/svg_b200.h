@@ -108,7 +108,7 @@ typedef struct svg_build_opts {
                                  share), 0 none (the default) */
     int32_t coop_warps;       /* warps that run them (0 automatic) */
     int32_t vote_wait;        /* batched: most loop iterations a lane waits for the warp's vote to pick its
-                                 kind of step (0 = 16) */
+                                 kind of step (0 = 16, or 8 at up to one block per SM) */
     int32_t heavy_waves;      /* batched: waves of lanes filled heaviest-first before vertex order (0 = 2) */
     int32_t heap_factor;      /* batched: first-pass physical window heap = heap_factor x K entries (0 = 3);
                                  a source that outgrows it is re-run with the full 1023 */

@@ -879,13 +879,6 @@ svg_build_opts effective_options(const svg_mesh* m, const svg_build_opts& o) {
                 e.coop_tail = t.opts.coop_tail;
             }
     }
-    // A lane's step is dearer the more lanes of its warp take it, and a step
-    // of one or two waiting lanes costs the others a whole step's latency: the
-    // rarer kinds are let gather for up to 16 steps.  Build kernel, ms, at 4 /
-    // 8 / 16 / 32: 5K vertices K=50 2.50 / 2.51 / 2.55 / 2.58, 30K K=100 14.1
-    // / 13.7 / 13.6 / 13.5, 72.9K K=500 425 / 409 / 401 / 404, 750K K=100 237 /
-    // 229 / 227 / 227.
-    if (e.vote_wait <= 0) e.vote_wait = 16;
     if (e.heavy_waves <= 0) e.heavy_waves = 2;
     if (e.heap_factor <= 0) e.heap_factor = 3;
     return e;
@@ -1231,7 +1224,6 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
     C.vref = (uint32_t)K * o.vert_coef;
     C.sref = (uint32_t)K * o.split_coef;
     C.watchdog = (int64_t)1 << 26;
-    C.max_wait = o.vote_wait;
     Layout lay;
     lay.wphys = C.wphys;
     lay.pphys = C.pphys;
@@ -1290,6 +1282,16 @@ svg_status build_once(svg_mesh* m, const svg_build_opts& o_in, svg_graph* g, int
         // lane: K = 500, 40K height field at one 424 / 517 ms, at two 300 /
         // 347 ms, 30K torus at one and a half 213 / 244 ms.
         const int64_t warps = (int64_t)blocks * (tpb / 32);
+        // A lane's step is dearer the more lanes of its warp take it, and a step
+        // of one or two waiting lanes costs the others a whole step's latency:
+        // the rarer kinds are let gather for up to 16 steps, or 8 at up to one
+        // block per SM, where few other warps fill the wait.  Build kernel, ms,
+        // at 4 / 8 / 16 / 32: 5K vertices K=50 2.50 / 2.51 / 2.55 / 2.58, 30K
+        // K=100 14.1 / 13.7 / 13.6 / 13.5, 72.9K K=500 425 / 409 / 401 / 404,
+        // 750K K=100 237 / 229 / 227 / 227; one block per SM at 4 / 8 / 16, 90K
+        // height field K=200 201 / 197 / 201, 40K 99.8 / 97.4 / 99.0, 150K torus
+        // 262 / 258 / 260, 30K 69.2 / 68.2 / 69.4 (K=50: within 0.5 %).
+        C.max_wait = o.vote_wait > 0 ? o.vote_wait : (warps > 4 * prop.multiProcessorCount ? 16 : 8);
         const bool equal = warps > 8 * prop.multiProcessorCount && (K >= 300 || (m->cost_K == K && m->cost_even));
         const int64_t waves = equal ? std::max<int64_t>(1, (nsrc + 32 * warps - 1) / (32 * warps)) : 1;
         warp_lanes = (int)std::max<int64_t>(1, std::min<int64_t>(32, (nsrc + warps * waves - 1) / (warps * waves)));
