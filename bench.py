@@ -1190,7 +1190,7 @@ def main():
         kw = dict(source_begin=sb, source_end=se) if shard else {}
         best, best_ms = svg.autotune(max_trials=16, **kw)
         tuned = {"params": {k: best[k] for k in ("coop_sources", "coop_warps", "blocks", "vote_wait",
-                                                 "heavy_waves", "heap_factor", "coop_tail")},
+                                                 "heavy_waves", "heap_factor")},
                  "tuned_build_ms": best_ms, "tuning_s": time.perf_counter() - t0}
     for _ in range(args.warmup):
         timed_build()
@@ -1292,10 +1292,11 @@ def main():
                                         if shard else f"replicas{ws}"),
                            edges_per_build=edges_per_build, windows_per_build=windows_per_build,
                            work_order="timed steps: the autotuned schedule (untimed tuning before the warm-up; "
-                                      "heaviest sources first, the heaviest on whole warps, by the per-source "
-                                      "costs the earlier builds recorded); e2e: a fresh mesh every step with the "
-                                      "default options (no cost record yet: on this mesh, under 4 sources per lane at "
-                                      "K >= 160, a K/10 probe build orders the sources)"),
+                                      "heaviest sources first by the per-source costs the earlier builds "
+                                      "recorded, the `autotune` field's number of them on whole warps); e2e: a "
+                                      "fresh mesh every step with the default options (no cost record yet: with "
+                                      "more than one and at most 8/3 sources per lane and K >= 160, as here, a "
+                                      "K/10 probe build orders the sources)"),
             "build_s": total_ms_max / args.steps / 1e3,
             "kernel_ms_per_step": statistics.mean(kern),
             "roofline": roofline_figures(st, peaks, fma_rate()),

@@ -225,8 +225,6 @@ __device__ void finish_warp(LaneType& L, const PhaseOut& O, int v, unsigned amas
     }
 }
 
-// Longest a lane waits for its action type to be chosen (iterations).
-
 // Persistent batched build.  Each lane runs one source at a time and pulls
 // the next from the device work queue.  Every iteration the warp votes: each
 // lane's next action is a window pop, a pseudo-source pop or "source done"
@@ -857,8 +855,7 @@ bool same_build_options(const svg_build_opts& a, const svg_build_opts& b) {
            a.threads_per_block == b.threads_per_block && a.blocks == b.blocks && a.with_paths == b.with_paths &&
            a.heavy_first == b.heavy_first && a.hbm_budget == b.hbm_budget && a.source_begin == b.source_begin &&
            a.source_end == b.source_end && a.coop_sources == b.coop_sources && a.coop_warps == b.coop_warps &&
-           a.vote_wait == b.vote_wait && a.heavy_waves == b.heavy_waves && a.heap_factor == b.heap_factor &&
-           a.coop_tail == b.coop_tail;
+           a.vote_wait == b.vote_wait && a.heavy_waves == b.heavy_waves && a.heap_factor == b.heap_factor;
 }
 }  // namespace
 
@@ -876,7 +873,6 @@ svg_build_opts effective_options(const svg_mesh* m, const svg_build_opts& o) {
                 e.heavy_waves = t.opts.heavy_waves;
                 e.heap_factor = t.opts.heap_factor;
                 e.blocks = t.opts.blocks;
-                e.coop_tail = t.opts.coop_tail;
             }
     }
     if (e.heavy_waves <= 0) e.heavy_waves = 2;
@@ -1778,7 +1774,6 @@ svg_status run_autotune(svg_mesh* m, const svg_build_opts& in, int32_t max_trial
     if (base.heavy_first == 0) base.heavy_first = 1;
     base.coop_sources = 0;
     base.coop_warps = 0;
-    base.coop_tail = 1;
     base.vote_wait = 16;
     base.heavy_waves = 2;
     base.heap_factor = 3;

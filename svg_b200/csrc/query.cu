@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kQThreads) k_query(QParams P) {
 }
 
 // ---------------------------------------------------------------------------
-// Team forms: one query per team of blocks, a thread-block cluster (8 or 16
+// Team forms: one query per team of blocks, a thread-block cluster (4, 8 or 16
 // blocks) or, for a few whole-graph searches, an equal share of every block
 // the GPU holds.  A batch runs only as many queries at once as there are
 // teams, so each query's distance and flag arrays stay in L2 while many SMs
