@@ -93,7 +93,8 @@ typedef struct svg_build_opts {
     int32_t pseudo_queue_cap; /* pseudo-source queue capacity (reference 1023) */
     int32_t mode;             /* svg_build_mode */
     int32_t threads_per_block;/* 0 = autotuned (batched) / 128 (plain, SVG.cuh:11) */
-    int32_t blocks;           /* 0 = autotuned (batched) / 64 (plain, SVG.cuh:10) */
+    int32_t blocks;           /* 0 = autotuned (batched) / 64 (plain, SVG.cuh:10); a batched build's retry pass
+                                 keeps to a given number too, unless full warps need more */
     int32_t with_paths;       /* 1 = also produce the path-end fields of svg_node */
     int32_t heavy_first;      /* batched, more sources than a launch's lanes: order the work queue heaviest
                                  first, by the per-source cost of the mesh's previous build at this K (1), or,
